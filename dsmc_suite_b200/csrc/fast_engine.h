@@ -2,8 +2,9 @@
 //
 // A fixed set of particle slots (one per resident thread) lives in HBM as structure-of-arrays.
 // Each launch advances every slot by up to K Verlet steps; a slot whose particle ends takes the
-// next particle from a device work queue that spans one or many problem instances. The launch
-// loop is captured once as a CUDA graph of G launches and replayed until the queue is drained.
+// next particle from a device work queue that spans one or many problem instances. A solve of one
+// instance launches kernels that carry its descriptor as a parameter; the served queue captures
+// its launch loop once as a CUDA graph of G launches and replays it.
 #pragma once
 
 #include <vector>
@@ -85,7 +86,104 @@ struct FastCounters {
     unsigned long long finished;  // particles whose life ended
     unsigned long long total;     // work items in the queue (sum of the instances' particles)
     long long ninst;              // instances in the queue
+    long long fill_warps;         // > 0: a queue of `total` particles, fewer than there are slots,
+                                  // starts on this many warps (particle w + l * fill_warps on
+                                  // lane l of warp w); 0: every slot takes from the queue
 };
+
+// The step loop's constants of one instance in the engine's precision.
+template <typename R>
+struct StepConst {
+    R GM, dt, c1, c2;        // FP32: GM dt, dt, 1.5 dt, dt / 6; FP64: GM, dt, 1.5 dt^2, dt^2 / 6
+    R rl2, re2;              // squared landing and escape radii
+    R fday, sx, sy, sz;      // weight factor of a day-side step, direction to the sun
+    float inv_bw;            // bins per m/s of the speed histogram
+    int flags, half_ffd, life_cap, hop_cap, col_ht, nbins;
+};
+enum StepFlag { kFlagRef = 1, kFlagSkipFirst = 2, kFlagCollide = 4, kFlagHist = 8 };
+
+template <typename R>
+__host__ __device__ inline StepConst<R> step_consts(const FastInst &I) {
+    const dsmc_params &p = I.p;
+    StepConst<R> k;
+    k.dt = static_cast<R>(p.dt_step);
+    if constexpr (sizeof(R) == sizeof(double)) {
+        k.GM = p.GM;
+        k.c1 = 1.5 * p.dt_step * p.dt_step;
+        k.c2 = p.dt_step * p.dt_step / 6.0;
+        k.rl2 = p.Radii * p.Radii;
+        k.re2 = p.max_height * p.max_height;
+    } else {
+        k.GM = static_cast<R>(p.GM * p.dt_step);
+        k.c1 = static_cast<R>(1.5 * p.dt_step);
+        k.c2 = static_cast<R>(p.dt_step / 6.0);
+        k.rl2 = I.r_land2;
+        k.re2 = I.r_esc2;
+    }
+    k.fday = static_cast<R>(p.wdecay);
+    k.sx = static_cast<R>(p.sun[0]);
+    k.sy = static_cast<R>(p.sun[1]);
+    k.sz = static_cast<R>(p.sun[2]);
+    k.half_ffd = p.ffd / 2;
+    k.flags = (p.model == DSMC_MODEL_REFERENCE ? kFlagRef : 0) |
+              (p.skip_first_deposit ? kFlagSkipFirst : 0) |
+              (p.runner == DSMC_RUNNER_ADVANCED && I.t.n_bg ? kFlagCollide : 0) |
+              (I.t.speed_hist && p.n_speed_bins > 0 ? kFlagHist : 0);
+    const long long most = 0x7fffffffLL, life = p.life_step_cap, hop = p.hop_step_cap;
+    k.life_cap = static_cast<int>(life <= 0 || life > most ? most : life);
+    k.hop_cap = static_cast<int>(hop > most ? most : hop);
+    k.col_ht = p.collide_ht_max;
+    k.nbins = p.n_speed_bins;
+    k.inv_bw = k.nbins > 0 ? static_cast<float>(1.0 / p.speed_bin_width) : 0.f;
+    return k;
+}
+
+// Kernel arguments. The queue's size (total work items, instances) is read from the counters.
+// FastArgsT: the served queue of many instances, whose descriptors lie in device memory.
+template <typename R>
+struct FastArgsT {
+    static constexpr bool kOne = false;
+    const FastInst *inst_;
+    SlotsT<R> s;
+    long long nslots;
+    FastCounters *ctr;
+    int K;
+    __device__ const FastInst &inst(int k) const { return inst_[k]; }
+    __device__ long long slot(long long i) const { return i; }
+};
+
+// OneArgsT: a solve of one instance, whose descriptor and step constants travel with the launch.
+// They lie in the constant bank, where an arithmetic instruction reads its operand for free: the
+// step loop keeps no constant in a register and an event reads its parameters without a load.
+template <typename R>
+struct OneArgsT {
+    static constexpr bool kOne = true;
+    FastInst one;
+    StepConst<R> k;
+    SlotsT<R> s;
+    long long nslots;
+    FastCounters *ctr;
+    int K;
+    const int *map;           // slot of each thread (-1: none), or nullptr: thread i has slot i
+    __device__ const FastInst &inst(int) const { return one; }
+    __device__ long long slot(long long i) const { return map ? map[i] : i; }
+};
+
+template <typename R> using OneKernel = void (*)(OneArgsT<R>);
+using ServedKernel = void (*)(FastArgsT<float>);
+// Steps in a row of the sparse loop (see fast_kernel).
+constexpr int kSparseUnroll = 8;
+// The kernels of a solve of one instance for a register budget of blocks_per_sm blocks of 128
+// threads (FP32: 4 or 5, FP64: 3 or 4); sparse: the loop for few particles, where the mode has one.
+OneKernel<float> one_kernel32(int blocks_per_sm, int mode, bool sparse);
+OneKernel<double> one_kernel64(int blocks_per_sm, int mode, bool sparse);
+// The kernels of a queue of many instances (fast_served.cu lists the variants).
+ServedKernel served_kernel(int variant, int mode);
+
+// Dynamic shared memory of a OneArgsT kernel: 256 columns (pairs), 256 rows, hd + 1 shells.
+inline size_t one_table_bytes(const dsmc_params &p, bool fp64) {
+    return (3 * 256 + static_cast<size_t>(p.hd) + 1) * (fp64 ? sizeof(double) : sizeof(float));
+}
 
 // Pieces of the engine for callers that supply every buffer themselves (no allocation here):
 // bytes of the slot arrays for nslots slots, of one instance descriptor and of the counters;
@@ -125,7 +223,6 @@ public:
                     long long n, int num_sms, cudaStream_t stream);
 
     void set_shape(int blk, int per_sm, int k, int g) {
-        if (blk != block || per_sm != blocks_per_sm) nslots_want_changed_ = true;
         block = blk;
         blocks_per_sm = per_sm;
         steps_per_launch = k;
@@ -142,15 +239,14 @@ public:
 
 private:
     cudaError_t ensure_slots(int num_sms);
-    cudaError_t upload_instances(const std::vector<dsmc_params> &ps,
-                                 const std::vector<DevTables> &ts,
-                                 const std::vector<long long> &counts,
-                                 const std::vector<long long> &pid_begins, cudaStream_t stream);
+    cudaError_t upload_one(const dsmc_params &p, const DevTables &t, long long pid_begin, long long n,
+                           cudaStream_t stream);
+    cudaError_t launch_one(cudaStream_t stream, long long threads, int steps, const int *map, bool sparse);
+    void launch_served(cudaStream_t stream, int mode, int steps);
     cudaError_t drain(long long total, cudaStream_t stream);
-    cudaError_t prepare_graph(cudaStream_t stream);
     cudaError_t capture(cudaStream_t stream, int mode, cudaGraphExec_t *out);
-    cudaError_t round(cudaStream_t stream);
-    void launch_kernel(cudaStream_t stream, int mode, unsigned grid);   // one launch, fp64_ state
+    long long warps_for(long long live) const;
+    void free_graphs();
 
 public:
     // Serving: an open queue that grows while it drains. serve_open resets the engine to an
@@ -199,15 +295,19 @@ private:
     int ninst_ = 0;
     float *d_tab_ = nullptr;
     size_t tab_cap_ = 0;
+    std::vector<float> tab_host_;             // staging of d_tab_
+    FastInst inst_host_{};                    // the instance of a solve
     FastCounters *d_ctr_ = nullptr;
-    FastCounters *h_ctr_ = nullptr;
-    cudaGraphExec_t graph_ = nullptr;
-    cudaGraphExec_t graph_mode_[3] = {nullptr, nullptr, nullptr};   // serving: lean loops 1, 2
-    cudaStream_t graph_stream_ = nullptr;
-    int graph_key_[4] = {0, 0, 0, 0};
-    bool nslots_want_changed_ = false;
-    int variant_ = 2;
-    int mode_ = 0;   // loop of run launches (see fast_kernel)
+    FastCounters *h_ctr_ = nullptr;           // [3] pinned: the last two launches', the start's
+    cudaEvent_t round_[2] = {nullptr, nullptr};
+    long long step_of_[2] = {0, 0};           // steps of the launches behind round_
+    int *d_map_ = nullptr;                    // packed slots of a drain's last launches
+    cudaGraphExec_t graph_mode_[3] = {nullptr, nullptr, nullptr};   // serving: loops 0, 1, 2
+    int num_sms_ = 0;
+    int variant_ = 4;
+    int mode_ = 0;            // loop of a solve (see Mode in fast_kernel.cuh)
+    bool one_ = false;        // a solve runs the kernels that take the instance with the launch
+    size_t one_smem_ = 0;     // their shared memory (the boundary tables)
 };
 
 }  // namespace dsmc

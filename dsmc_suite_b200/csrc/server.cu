@@ -33,7 +33,7 @@
 namespace {
 
 using Clock = std::chrono::steady_clock;
-constexpr int kSnapHead = 4;   // words of FastCounters at the start of a snapshot
+constexpr int kSnapHead = 5;   // words of FastCounters at the start of a snapshot
 
 struct Request {
     long long n = 0;

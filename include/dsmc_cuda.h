@@ -94,7 +94,8 @@ typedef struct dsmc_ctx dsmc_ctx;
  * boundary tables (no compensation needed), with the plain path's FP64 maps of the random words
  * at launches and collisions: it follows the same Philox streams as PLAIN_FP64 and differs from
  * it only by rounding, so it serves as the full-size FP64 reference of FAST_FP32. FAST_FP64
- * runs 128-thread blocks, 4 (default) or 3 resident per SM. */
+ * runs 128-thread blocks, 5 resident per SM in its lean loop (config model, ballistic, no speed
+ * histogram), else 4 (3 when asked). */
 enum dsmc_path { DSMC_PATH_PLAIN_FP64 = 0, DSMC_PATH_FAST_FP32 = 1, DSMC_PATH_FAST_FP64 = 2 };
 
 typedef struct dsmc_stats {
@@ -128,8 +129,9 @@ int dsmc_run(dsmc_ctx *ctx, int path, int64_t pid_begin, int64_t n);
 int dsmc_sync(dsmc_ctx *ctx);
 
 /* Launch shape of the FAST paths: threads per block, resident blocks per SM (0 = as many as
- * fit), Verlet steps per slot per launch, and launches per captured CUDA graph (1 = no graph).
- * Results do not depend on the shape: every particle's trajectory is a function of its id and
+ * fit), Verlet steps per slot per launch (the last launches of a solve are shorter), and launches
+ * per captured CUDA graph (served rounds; a solve's launches carry its parameters and are issued
+ * one by one). Results do not depend on the shape: every particle's trajectory is a function of its id and
  * the deposits are integer sums. */
 int dsmc_set_launch_shape(dsmc_ctx *ctx, int block, int blocks_per_sm, int steps_per_launch,
                           int launches_per_graph);

@@ -1,0 +1,57 @@
+"""A solve of one instance against the kernels of the served queue (needs a B200).
+
+A solve in the default launch shape runs loops that take the instance with the launch, start few
+particles on a lane spread, switch to the sparse loop below a particle count and pack the live
+slots once the queue is empty; a 256-thread shape runs the general loops of the served queue over
+descriptors in device memory. A particle's trajectory, random stream and deposits are functions of
+its id alone, so both give the same grids, rows and counters bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from conftest import cold_T
+
+pytestmark = pytest.mark.gpu
+
+BODIES = {"ceres": (470e3, 6.26e10), "moon": (1737e3, 4.90e12)}
+# edges of a warp, of one warp per scheduler, of the sparse loop's range and of the slots (640 per
+# SM), on a GPU of 148 SMs
+SIZES = [1, 33, 593, 59_200, 59_201, 94_719, 94_721, 200_003]
+
+
+def _problem(N, kind):
+    if kind == "reference":
+        p = N.params_reference(N.RUNNER_BALLISTIC, 36, 72)
+        return p, N.SurfaceInputs(T_map=cold_T(N))
+    R, GM = BODIES[kind.split("_")[0]]
+    p = N.params_config(N.RUNNER_BALLISTIC, R, GM, 41, 77)
+    if kind.endswith("_hist"):
+        p.n_speed_bins = 24
+        p.speed_bin_width = 40.0
+    if kind.endswith("_cap"):   # the hop cap below the life cap: the general loop
+        p.hop_step_cap = 111
+    ico = N.Icosphere(3)
+    return p, N.SurfaceInputs(ico=ico, face_T=ico.face_temperature())
+
+
+@pytest.mark.parametrize("kind,n", [(k, n) for k in ("ceres", "moon") for n in SIZES] +
+                         [(k, n) for k in ("ceres_hist", "ceres_cap") for n in (33, 94_721)] +
+                         [("reference", n) for n in (33, 5_000)])
+def test_one_instance_equals_served_kernels(N, kind, n):
+    from dsmc_suite_b200 import Context
+    p, S = _problem(N, kind)
+    res = []
+    for shape in (None, (256, 2, 3000, 2)):
+        with Context(0) as ctx:
+            if shape:
+                ctx.set_launch_shape(*shape)
+            r = ctx.solve(N.PATH_FAST_FP32, p, S, n, outputs=True)
+            if p.n_speed_bins:
+                r["hist"] = ctx.speed_hist()
+            res.append(r)
+    a, b = res
+    assert a["stats"] == b["stats"] and a["stats"]["n_finished"] == n
+    for key in a:
+        if key != "stats":
+            assert np.array_equal(a[key], b[key]), key
