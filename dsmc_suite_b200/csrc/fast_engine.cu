@@ -186,15 +186,15 @@ cudaError_t FastEngine::ensure_slots(int num_sms) {
 
 namespace {
 
-// Steps of a launch once the queue is nearly empty. On 3e5 Ceres-like particles 4096 runs in
-// 14.6 ms against 15.1 ms at 2048 and 16.6 ms at 1024 (a launch ends with its slowest warp).
-constexpr int kTailSteps = 4096;
+// Idle limit (lane-chunks) of event gathering once the live slots are packed: a lane that waits
+// then delays the end of the solve. 1e6 Europa-like particles in FP64 ran 25.7 ms at the full
+// limit of 16, 25.1 ms at 2 and 25.4 ms at 0; 3e5 Moon-like 8.6, 8.25 and 8.4 ms.
+constexpr int kTailGather = 2;
 
-// A solve of at most this many particles per SM runs the sparse loop: 5e4 Moon-like particles
-// (340 per SM) take 4.1 ms against 5.4 ms in the bulk loop, 1e4 Ceres-like 2.3 ms against
-// 3.8 ms. The tail of a larger solve keeps the bulk loop: its survivors are the long-lived
-// particles, which cross cells and land so often that the sparse loop's longer slow path loses
-// (3e5 Ceres-like: 14.6 ms against 15.2 ms with the sparse loop below 120 lanes per SM).
+// A launch over at most this many live particles per SM runs the sparse loop: 5e4 Moon-like
+// particles (340 per SM) take 3.9 ms against 5.4 ms in the bulk loop, 1e4 Ceres-like 2.3 ms
+// against 3.8 ms, and in the tail of larger solves 3e5 Moon-like 7.0 ms against 8.4 ms, 3e5
+// Ceres-like 10.9 against 12.5 ms (200 to 500 per SM are within 1 %).
 constexpr int kSparsePerSm = 400;
 
 // Warps per SM that a few particles are spread over: one per scheduler. More warps of fewer lanes
@@ -327,7 +327,7 @@ cudaError_t FastEngine::upload_one(const dsmc_params &p, const DevTables &t, lon
 }
 
 // One launch of the solve's kernel over `threads` slots (map: see drain).
-cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, int steps, const int *map, bool sparse) {
+cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, const int *map, bool sparse) {
     const unsigned grid = static_cast<unsigned>(threads / block);   // whole blocks (see warps_for)
     auto fill = [&](auto &a, const auto &slots) {
         a.one = inst_host_;
@@ -335,8 +335,9 @@ cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, int s
         a.s = slots;
         a.nslots = nslots_;
         a.ctr = d_ctr_;
-        a.K = steps;
+        a.K = steps_per_launch;
         a.map = map;
+        a.gather = map ? std::min(inst_host_.gather, kTailGather) : inst_host_.gather;
     };
     if (slot_fp64_) {
         OneArgsT<double> a{};
@@ -347,19 +348,19 @@ cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, int s
         fill(a, slots_);
         one_kernel32(variant_, mode_, sparse)<<<grid, block, one_smem_, stream>>>(a);
     } else {
-        launch_served(stream, mode_ <= 2 ? mode_ : 0, steps);
+        launch_served(stream, mode_ <= 2 ? mode_ : 0);
     }
     return cudaGetLastError();
 }
 
 // One launch of a served loop over every slot.
-void FastEngine::launch_served(cudaStream_t stream, int mode, int steps) {
+void FastEngine::launch_served(cudaStream_t stream, int mode) {
     FastArgsT<float> a{};
     a.inst_ = d_inst_;
     a.s = slots_;
     a.nslots = nslots_;
     a.ctr = d_ctr_;
-    a.K = steps;
+    a.K = steps_per_launch;
     served_kernel(variant_, mode)<<<static_cast<unsigned>(nslots_ / block), block, 0, stream>>>(a);
 }
 
@@ -369,7 +370,7 @@ cudaError_t FastEngine::capture(cudaStream_t stream, int mode, cudaGraphExec_t *
     cudaGraph_t g;
     *out = nullptr;
     if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
-    for (int k = 0; k < launches_per_graph; k++) launch_served(stream, mode, steps_per_launch);
+    for (int k = 0; k < launches_per_graph; k++) launch_served(stream, mode);
     if ((e = cudaStreamEndCapture(stream, &g)) != cudaSuccess) return e;
     e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
@@ -379,11 +380,11 @@ cudaError_t FastEngine::capture(cudaStream_t stream, int mode, cudaGraphExec_t *
 
 // Launches until every particle of the queue has finished.
 //
-// While the queue still holds many launches' worth of particles, launches of steps_per_launch
-// steps run back to back, the host reading the counters of one while the next runs. Near the end
-// of the queue the launches get shorter and the host waits for each: once the queue is empty the
-// slots drain unevenly, and before each launch the live ones are packed over as few warps as
-// keep every scheduler busy (pack_slots_kernel), so that no warp is issued for a few lanes.
+// While the queue still holds several launches' worth of particles the launches run back to back,
+// the host reading the counters of one while the next runs. Near the end of the queue the host
+// waits for each: once the queue is empty the slots drain unevenly, and before each launch the
+// live ones are packed over as few warps as keep every scheduler busy (pack_slots_kernel), so
+// that no warp is issued for a few lanes.
 cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
     cudaError_t e;
     launches = 0;
@@ -399,8 +400,6 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
     int *inst = slot_fp64_ ? slots64_.inst : slots_.inst;
     if ((e = cudaMemsetAsync(inst, 0xff, nslots_ * sizeof(int), stream)) != cudaSuccess) return e;
     const long long whole = start->fill_warps ? start->fill_warps * 32 : nslots_;
-    const long long short_steps = std::min(steps_per_launch, kTailSteps);
-    const bool sparse = total <= static_cast<long long>(kSparsePerSm) * num_sms_;
     // Every launch advances each live particle by its steps or ends it, and every life is bounded
     // by its step caps, so the queue drains. The loop still gives up (launch-timeout status) if
     // no particle finishes for 2^28 steps, which would mean a logic error, not a long solve.
@@ -410,7 +409,6 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
     for (;;) {
         const double left = rate > 0.0 ? (static_cast<double>(total) - static_cast<double>(next)) / rate : 0.0;
         const bool empty = next >= static_cast<unsigned long long>(total);
-        const long long steps = left > 2.0 * steps_per_launch ? steps_per_launch : short_steps;
         long long threads = whole;
         const int *map = nullptr;
         if (one_ && empty && live < whole) {
@@ -421,11 +419,10 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
             threads = w * 32;
             map = d_map_ + 32;
         }
-        if ((e = launch_one(stream, threads, static_cast<int>(steps), map, sparse)) != cudaSuccess)
+        if ((e = launch_one(stream, threads, map, live <= static_cast<long long>(kSparsePerSm) * num_sms_)) != cudaSuccess)
             return e;
         launches++;
         const int at = static_cast<int>(issued & 1);
-        step_of_[at] = steps;
         if ((e = cudaMemcpyAsync(h_ctr_ + at, d_ctr_, sizeof(FastCounters), cudaMemcpyDeviceToHost, stream)) != cudaSuccess ||
             (e = cudaEventRecord(round_[at], stream)) != cudaSuccess)
             return e;
@@ -437,8 +434,8 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
             seen++;
             const FastCounters &c = h_ctr_[r];
             if (c.finished >= static_cast<unsigned long long>(total)) return cudaStreamSynchronize(stream);
-            rate = static_cast<double>(c.next - next) / static_cast<double>(step_of_[r]);
-            quiet = c.finished == finished ? quiet + step_of_[r] : 0;
+            rate = static_cast<double>(c.next - next) / steps_per_launch;
+            quiet = c.finished == finished ? quiet + steps_per_launch : 0;
             next = c.next;
             finished = c.finished;
             live = total - static_cast<long long>(finished);
@@ -573,7 +570,7 @@ cudaError_t FastEngine::serve_launch(cudaStream_t stream, int mode) {
         if (e == cudaSuccess) launches += launches_per_graph;
         return e;
     }
-    launch_served(stream, mode, steps_per_launch);
+    launch_served(stream, mode);
     const cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) launches += 1;
     return e;

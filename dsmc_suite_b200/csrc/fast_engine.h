@@ -164,6 +164,7 @@ struct OneArgsT {
     long long nslots;
     FastCounters *ctr;
     int K;
+    int gather;               // lane-chunks of event gathering in this launch (see fast_kernel)
     const int *map;           // slot of each thread (-1: none), or nullptr: thread i has slot i
     __device__ const FastInst &inst(int) const { return one; }
     __device__ long long slot(long long i) const { return map ? map[i] : i; }
@@ -241,8 +242,8 @@ private:
     cudaError_t ensure_slots(int num_sms);
     cudaError_t upload_one(const dsmc_params &p, const DevTables &t, long long pid_begin, long long n,
                            cudaStream_t stream);
-    cudaError_t launch_one(cudaStream_t stream, long long threads, int steps, const int *map, bool sparse);
-    void launch_served(cudaStream_t stream, int mode, int steps);
+    cudaError_t launch_one(cudaStream_t stream, long long threads, const int *map, bool sparse);
+    void launch_served(cudaStream_t stream, int mode);
     cudaError_t drain(long long total, cudaStream_t stream);
     cudaError_t capture(cudaStream_t stream, int mode, cudaGraphExec_t *out);
     long long warps_for(long long live) const;
@@ -300,7 +301,6 @@ private:
     FastCounters *d_ctr_ = nullptr;
     FastCounters *h_ctr_ = nullptr;           // [3] pinned: the last two launches', the start's
     cudaEvent_t round_[2] = {nullptr, nullptr};
-    long long step_of_[2] = {0, 0};           // steps of the launches behind round_
     int *d_map_ = nullptr;                    // packed slots of a drain's last launches
     cudaGraphExec_t graph_mode_[3] = {nullptr, nullptr, nullptr};   // serving: loops 0, 1, 2
     int num_sms_ = 0;

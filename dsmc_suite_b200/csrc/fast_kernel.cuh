@@ -415,9 +415,10 @@ __device__ __forceinline__ R c_day_of(const FastInst &I) {
 // shared boundary from the registers and loads only the next one, so a typical crossing costs
 // one table load. Same cells as track_shell / track_angles. in_r, in_t, in_f are the step's own
 // inside tests per coordinate; only the coordinates that failed are walked (7 % faster on
-// the 1e8-particle Ceres-like workload than walking all three, identical cells).
+// the 1e8-particle Ceres-like workload than walking all three, identical cells). Returns whether
+// the cell changed.
 template <bool kNoBg, class T, typename R>
-__device__ __forceinline__ void move_cell(const T &tab, HotT<R> &h, BoundsT<R> &b, R x, R y,
+__device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &b, R x, R y,
                                           R r2, R zz, bool in_r, bool in_t, bool in_f) {
     const FastInst &I = tab.I;
     int ht = h.cell >> 16, td = (h.cell >> 8) & 0xff, fd = h.cell & 0xff;
@@ -482,7 +483,7 @@ __device__ __forceinline__ void move_cell(const T &tab, HotT<R> &h, BoundsT<R> &
         }
     }
     const int cell = pack_cell(ht, td, fd);
-    if (cell == h.cell) return;
+    if (cell == h.cell) return false;
     // the run of a flying particle has a cell and no negative weight: flushed without the tests
     // of flush_cell (a run of zero adds zero)
     atomicAdd(&I.t.density[h.ci], fixed_of(h.run_w));
@@ -495,6 +496,7 @@ __device__ __forceinline__ void move_cell(const T &tab, HotT<R> &h, BoundsT<R> &
         if (I.p.runner == DSMC_RUNNER_ADVANCED && ht < I.p.collide_ht_max && h.ci < I.t.n_bg_len)
             h.nsig = static_cast<R>(__ldg(I.t.n_bg + h.ci) * I.p.cross_section);
     }
+    return true;
 }
 
 __device__ __forceinline__ double cdf_eval(const double *coef, const double *box, int degree,
@@ -1327,6 +1329,19 @@ __device__ __forceinline__ void count_speed(const FastInst &I, const StepConst<R
     }
 }
 
+// The rest of a segment of a particle whose position is not a number (a launch draw of exactly 1
+// in FP32, about once in 1e7 launches, gives it an infinite speed): every test of every step is
+// false, so it stays in its cell, outside the day side, and deposits its weight until the segment
+// ends. Stepping it instead sent it through the cell walk on every step, 0.37 us a step, which
+// was the length of a whole solve of 3e5 Moon-like particles (10.7 ms with such a particle, 8.6 ms
+// without). Returns the steps taken; the deposits are summed one by one, as the loop would.
+template <typename R>
+__device__ __forceinline__ int drift_nowhere(HotT<R> &h, int taken, int n) {
+    h.run_w += h.W;   // the step that found it
+    for (; taken < n; taken++) h.run_w += h.W;
+    return taken;
+}
+
 // kMaxThreads x kMinBlocks: the register budget the allocation must respect (65536 registers
 // per SM shared by kMinBlocks blocks of kMaxThreads). The launch shape picks the variant.
 // kMode: see Mode. A: the queue (FastArgsT) or one instance (OneArgsT). R: float (FAST_FP32) or
@@ -1410,8 +1425,9 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
         // together. Long hops (Ceres-like) keep the free-running loop. The limit is the largest
         // of the instances of the lanes that enter the segment together, so it is uniform.
         const unsigned peers = __activemask();
-        const int limit = A::kOne ? I.gather
-                                  : static_cast<int>(__reduce_max_sync(peers, static_cast<unsigned>(I.gather)));
+        int limit;
+        if constexpr (A::kOne) limit = a.gather;
+        else limit = static_cast<int>(__reduce_max_sync(peers, static_cast<unsigned>(I.gather)));
         const bool gather = limit > 0;
         const int npeer = __popc(peers);
         int idle = 0;
@@ -1456,7 +1472,11 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f);
+                if (!move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                    q.r2 != q.r2) {
+                    taken = drift_nowhere(h, taken, n);
+                    break;
+                }
                 settle();
             }
         }
@@ -1484,7 +1504,11 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                move_cell<!M::kAny && !M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f);
+                if (!move_cell<!M::kAny && !M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f) &&
+                    kMode == 1 && q.r2 != q.r2) {
+                    taken = drift_nowhere(h, taken, n);
+                    break;
+                }
             }
             const bool day = M::kRef || (M::kAny && (k.flags & kFlagRef))
                                  ? ((h.cell & 0xff) < k.half_ffd)

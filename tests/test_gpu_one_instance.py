@@ -55,3 +55,33 @@ def test_one_instance_equals_served_kernels(N, kind, n):
     for key in a:
         if key != "stats":
             assert np.array_equal(a[key], b[key]), key
+
+
+def test_particle_without_a_position(N):
+    """Two particles of one stream draw an infinite launch speed (an FP32 uniform of exactly 1),
+    one at its first launch, one after 23 hops: from then on each deposits its weight into the cell
+    it launched from until its life cap. The first has unit weight, so its deposit is known; the
+    second is compared with the general loop, which steps such a particle like any other."""
+    from dsmc_suite_b200 import Context
+    R, GM = BODIES["moon"]
+    p = N.params_config(N.RUNNER_BALLISTIC, R, GM, 50, 20261203)
+    ico = N.Icosphere(3)
+    S = N.SurfaceInputs(ico=ico, face_T=ico.face_temperature())
+
+    def one(pid, hop_cap):
+        q = p.copy()
+        q.hop_step_cap = hop_cap
+        with Context(0) as ctx:
+            ctx.setup(q, S)
+            ctx.enable_particle_outputs(1)
+            ctx.run(N.PATH_FAST_FP32, pid, 1)
+            ctx.sync()
+            ttime, _, steps = ctx.particle_outputs(1)
+            assert np.isnan(ttime[1, 0]) and steps[0] == 20_000
+            return ctx.density(), ttime[3, 0]
+
+    d, w = one(287_594, 20_000)
+    assert w == 1.0 and d[0, 22, 48] == 20_000 << 24 and np.count_nonzero(d) == 1
+    a, wa = one(200_964, 20_000)
+    b, wb = one(200_964, 19_999)   # a hop cap below the life cap: the general loop
+    assert wa == wb < 1.0 and np.array_equal(a, b)
