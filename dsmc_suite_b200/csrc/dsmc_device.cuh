@@ -18,6 +18,9 @@ enum StatSlot { kStatSteps = 0, kStatEscaped, kStatCollisions, kStatBound, kStat
 struct DevTables {
     // reference model
     const double *T_map;          // [ftd][ffd]
+    const int *warm;              // [ftd][ffd] rotation steps a frozen particle waits in a cell for
+                                  // the first column at or above freeze_T (0: none in its row),
+                                  // or nullptr: scan T_map
     const double *vt_speeds;      // [23][1000], velocity table of src/common/velocity.c:6-47
     const int *vt_count;          // [23]
     // config model

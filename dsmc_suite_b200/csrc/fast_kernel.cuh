@@ -839,6 +839,20 @@ __device__ __forceinline__ R column_centre(int fd, int ffd) {
     else return (fd + 0.5f) / ffd * 2.0f * kPiF;
 }
 
+// Turns the position by `cols` columns of longitude (the advanced runner's freeze scan,
+// advanced.c:290-300).
+template <typename R>
+__device__ __forceinline__ void turn_to_column(HotT<R> &h, int cols, int ffd) {
+    const double rot_fi = static_cast<double>(cols) / ffd * 2.0 * kPi;
+    const double cs = cos(rot_fi), sn = sin(rot_fi);
+    double s[3];
+    get_pos(h, s);
+    const double n0 = s[0] * cs - s[1] * sn, n1 = s[0] * sn + s[1] * cs;
+    s[0] = n0;
+    s[1] = n1;
+    set_pos(h, s);
+}
+
 // Start of a hop (ballistic.c:124-181, advanced.c:271-333): weight and life checks, the
 // reference freeze scan, the launch and the starting cell. Returns 0 when the particle flies,
 // else its fate.
@@ -858,7 +872,21 @@ __device__ __forceinline__ int hop_top(const A &a, long long i, const FastInst &
         if (local_T < static_cast<R>(p.freeze_T)) {
             bool found = false;
             float rest = a.s.rest[i];
-            if (p.runner == DSMC_RUNNER_BALLISTIC) {
+            if (I.t.warm) {
+                if (p.runner != DSMC_RUNNER_BALLISTIC) horizon_add(I, td, fd, W);
+                const int wait = I.t.warm[td * ffd + fd];
+                for (int k = wait ? wait : ffd; k > 0; k--) rest += static_cast<float>(p.dt_rot);
+                if (wait) {
+                    found = true;
+                    if (p.runner == DSMC_RUNNER_BALLISTIC) {
+                        fd = (fd + wait) % ffd;
+                    } else {
+                        turn_to_column(h, wait - fd, ffd);
+                        fd = wait % ffd;
+                    }
+                    fi = column_centre<R>(fd, ffd);
+                }
+            } else if (p.runner == DSMC_RUNNER_BALLISTIC) {
                 for (int add = 0; add < ffd; add++) {
                     rest += static_cast<float>(p.dt_rot);
                     const int check = (fd + add + 1) % ffd;
@@ -874,14 +902,7 @@ __device__ __forceinline__ int hop_top(const A &a, long long i, const FastInst &
                 for (int add = 1; add <= ffd; add++) {
                     rest += static_cast<float>(p.dt_rot);
                     if (T[td * ffd + (add % ffd)] >= p.freeze_T) {
-                        const double rot_fi = static_cast<double>(add - fd) / ffd * 2.0 * kPi;
-                        const double cs = cos(rot_fi), sn = sin(rot_fi);
-                        double s[3];
-                        get_pos(h, s);
-                        const double n0 = s[0] * cs - s[1] * sn, n1 = s[0] * sn + s[1] * cs;
-                        s[0] = n0;
-                        s[1] = n1;
-                        set_pos(h, s);
+                        turn_to_column(h, add - fd, ffd);
                         fd = add % ffd;
                         fi = column_centre<R>(fd, ffd);
                         found = true;

@@ -151,7 +151,24 @@ __device__ void particle_life(const dsmc_params &p, const DevTables &t, long lon
             local_T = t.T_map[td * ffd + fd];
             if (local_T < p.freeze_T) {
                 bool found = false;
-                if (!adv) {
+                if (t.warm) {
+                    if (adv && kMode == kSolve) atomicAdd(&t.horizon[td * ffd + fd], to_fixed(W));
+                    const int wait = t.warm[td * ffd + fd];
+                    for (int k = wait ? wait : ffd; k > 0; k--) {
+                        time += p.dt_rot;
+                        if (adv) rest_time += p.dt_rot;
+                    }
+                    if (wait) {
+                        found = true;
+                        if (adv) {
+                            turn_to_column(s, wait - fd, ffd);
+                            fd = wait % ffd;
+                        } else {
+                            fd = (fd + wait) % ffd;
+                        }
+                        fi = (fd + 0.5) / ffd * 2.0 * kPi;
+                    }
+                } else if (!adv) {
                     for (int add = 0; add < ffd; add++) {
                         time += p.dt_rot;
                         const int check = (fd + add + 1) % ffd;
@@ -168,11 +185,7 @@ __device__ void particle_life(const dsmc_params &p, const DevTables &t, long lon
                         time += p.dt_rot;
                         rest_time += p.dt_rot;
                         if (t.T_map[td * ffd + (add % ffd)] >= p.freeze_T) {
-                            const double rot_fi = static_cast<double>(add - fd) / ffd * 2.0 * kPi;
-                            const double cs = cos(rot_fi), sn = sin(rot_fi);
-                            const double n0 = s[0] * cs - s[1] * sn, n1 = s[0] * sn + s[1] * cs;
-                            s[0] = n0;
-                            s[1] = n1;
+                            turn_to_column(s, add - fd, ffd);
                             fd = add % ffd;
                             fi = (fd + 0.5) / ffd * 2.0 * kPi;
                             found = true;

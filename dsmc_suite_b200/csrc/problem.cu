@@ -2,6 +2,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "problem.h"
 
@@ -26,6 +27,29 @@ const VelocityTable &speed_table() {
 int report(char *err, size_t n, int status, const char *what, cudaError_t e) {
     if (err && n) std::snprintf(err, n, "%s: %s", what, cudaGetErrorString(e));
     return status;
+}
+
+// The freeze scans of the reference (ballistic.c:132-153, advanced.c:278-309) as a table: the
+// rotation steps until the first warm column, counted from the particle's own column (ballistic)
+// or from column 0 (advanced), 0 where the row has none. The scan read up to ffd map entries one
+// after the other at every launch from a cold cell.
+std::vector<int> warm_table(const dsmc_params &p, const double *T) {
+    std::vector<int> w(static_cast<size_t>(p.ftd) * p.ffd);
+    for (int td = 0; td < p.ftd; td++) {
+        const double *row = T + static_cast<size_t>(td) * p.ffd;
+        int *out = w.data() + static_cast<size_t>(td) * p.ffd;
+        // steps from each column to the next warm one, walking twice round the row backwards
+        int next = 0;
+        for (int k = 2 * p.ffd - 1; k >= 0; k--) {
+            const int fd = k % p.ffd;
+            if (k < p.ffd) out[fd] = next;
+            if (row[fd] >= p.freeze_T) next = 1;
+            else if (next) next++;
+        }
+        if (p.runner != DSMC_RUNNER_BALLISTIC)
+            for (int fd = p.ffd - 1; fd >= 0; fd--) out[fd] = out[0];
+    }
+    return w;
 }
 
 struct Uploader {
@@ -90,7 +114,7 @@ size_t problem_bytes(const dsmc_params *p, const dsmc_surface *s, const dsmc_col
     size_t b = (ncell + nh) * 8;
     if (p->n_speed_bins > 0) b += ncell * p->n_speed_bins * 8;
     if (p->model == DSMC_MODEL_REFERENCE) {
-        b += nh * 8 + 23 * 1000 * 8 + 23 * 4;
+        b += nh * (8 + 4) + 23 * 1000 * 8 + 23 * 4;
     } else if (s) {
         const size_t nf = static_cast<size_t>(s->nface), nn = static_cast<size_t>(20 * ((1 << (2 * s->nlevel)) - 1) / 3);
         b += nf * 9 * 8 + nf * 8 * (s->face_cdf ? 2 : 1) + 60 * 8 + nn * 9 * 8;
@@ -153,6 +177,10 @@ int problem_build(Problem &pr, const dsmc_params *p, const dsmc_surface *s,
         const double *d_T = nullptr, *d_sp = nullptr;
         const int *d_cnt = nullptr;
         if ((rc = u.upload(s->T_map, static_cast<size_t>(ftd * ffd), &d_T)) != DSMC_OK) return rc;
+        const std::vector<int> warm = warm_table(*p, s->T_map);
+        const int *d_warm = nullptr;
+        if ((rc = u.upload(warm.data(), warm.size(), &d_warm)) != DSMC_OK) return rc;
+        t.warm = d_warm;
         if ((rc = u.upload(&vt.speeds[0][0], 23 * 1000, &d_sp)) != DSMC_OK) return rc;
         if ((rc = u.upload(vt.count, 23, &d_cnt)) != DSMC_OK) return rc;
         t.T_map = d_T;
