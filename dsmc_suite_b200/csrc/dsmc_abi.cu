@@ -656,12 +656,13 @@ int dsmc_velocity_record(dsmc_ctx *c, int64_t n, int per_bucket, int64_t total_c
     if (rc != DSMC_OK) return rc;
     const int hd = c->params.hd;
     const long long nb = static_cast<long long>(c->params.ftd) * hd;
-    // Chunk of particles whose per-bucket counter rows fit in ~64 MB.
-    long long chunk = (64ll << 20) / (4 * nb);
+    // Chunk of particles whose per-bucket counter rows fit in ~256 MB (a chunk takes as long as its
+    // longest-lived particle, so few large ones).
+    long long chunk = (256ll << 20) / (4 * nb);
     chunk = chunk < 256 ? 256 : chunk;
     if (chunk > n) chunk = n > 0 ? n : 1;
     struct Bufs {
-        void *p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+        void *p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
         ~Bufs() { for (void *q : p) if (q) cudaFree(q); }
     } b;
     const long long slots = nb * per_bucket;
@@ -670,10 +671,12 @@ int dsmc_velocity_record(dsmc_ctx *c, int64_t n, int per_bucket, int64_t total_c
     DSMC_CUDA_TRY(c, cudaMalloc(&b.p[2], slots * 3 * sizeof(double)));
     DSMC_CUDA_TRY(c, cudaMalloc(&b.p[3], slots * sizeof(int)));
     DSMC_CUDA_TRY(c, cudaMalloc(&b.p[4], slots * sizeof(unsigned long long)));
+    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[5], chunk * sizeof(int)));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(b.p[1], 0, nb * sizeof(int), c->stream));
     dsmc::RecordArgs ra{};
     ra.rows = static_cast<int *>(b.p[0]);
     ra.cap = per_bucket;
+    ra.todo = static_cast<int *>(b.p[5]);
     ra.rec_v = static_cast<double *>(b.p[2]);
     ra.rec_fd = static_cast<int *>(b.p[3]);
     ra.rec_key = static_cast<unsigned long long *>(b.p[4]);

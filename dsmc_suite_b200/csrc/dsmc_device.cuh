@@ -38,6 +38,9 @@ struct DevTables {
     const double *cdf_total;      // [ncell]
     const int *cdf_valid;         // [ncell]
     int cdf_degree;
+    // cell edges for the plain FP64 path (cell_edges in problem.cu), or nullptr: radii [hd+1], sines
+    // of the latitudes [ftd+1], (sine, cosine) of the longitudes [ffd+1][2]
+    const double *edges;
     // outputs
     unsigned long long *density;  // [hd][ftd][ffd] fixed point
     unsigned long long *horizon;  // [ftd][ffd] fixed point
@@ -54,6 +57,7 @@ struct DevTables {
 struct RecordArgs {
     int *rows;                    // [chunk][ftd*hd]
     long long row_base;           // pid of row 0
+    int *todo;                    // [chunk] records of each particle that fall below the cap
     int cap;                      // records per bucket (200 in the reference)
     double *rec_v;                // [ftd*hd][cap][3]
     int *rec_fd;                  // [ftd*hd][cap]

@@ -1,4 +1,5 @@
 // problem.cu - upload of one DSMC problem to the device (see problem.h).
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -50,6 +51,21 @@ std::vector<int> warm_table(const dsmc_params &p, const double *T) {
             for (int fd = p.ffd - 1; fd >= 0; fd--) out[fd] = out[0];
     }
     return w;
+}
+
+// Edges of the grid cells as the index formulas place them (grid.c:28-39, grid.c:91-99): shell k
+// starts where log(alpha2 (r - R) / unih + 1) / log1p_alpha2 = k, or at R + k unih.
+std::vector<double> cell_edges(const dsmc_params &p) {
+    std::vector<double> e;
+    for (int k = 0; k <= p.hd; k++)
+        e.push_back(p.use_exp_grid ? p.Radii + p.unih * (std::exp(k * p.log1p_alpha2) - 1.0) / p.alpha2
+                                   : p.Radii + k * p.unih);
+    for (int k = 0; k <= p.ftd; k++) e.push_back(std::sin((static_cast<double>(k) / p.ftd - 0.5) * kPi));
+    for (int k = 0; k <= p.ffd; k++) {
+        e.push_back(std::sin(2.0 * kPi * k / p.ffd));
+        e.push_back(std::cos(2.0 * kPi * k / p.ffd));
+    }
+    return e;
 }
 
 struct Uploader {
@@ -219,6 +235,10 @@ int problem_build(Problem &pr, const dsmc_params *p, const dsmc_surface *s,
         t.cdf_total = ct;
         t.cdf_valid = cv;
         t.cdf_degree = col->cdf_degree;
+    }
+    if (!async_alloc) {   // served requests run the FAST engine only
+        const std::vector<double> edges = cell_edges(*p);
+        if ((rc = u.upload(edges.data(), edges.size(), &t.edges)) != DSMC_OK) return rc;
     }
     if ((rc = u.zeroed(static_cast<size_t>(pr.ncell), &t.density)) != DSMC_OK) return rc;
     if ((rc = u.zeroed(static_cast<size_t>(pr.nhcell), &t.horizon)) != DSMC_OK) return rc;

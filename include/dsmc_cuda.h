@@ -87,7 +87,8 @@ int dsmc_source_cdf(int nface, const double *face_verts, const double *face_T, d
 typedef struct dsmc_ctx dsmc_ctx;
 
 /* Solve paths. PLAIN_FP64 is the straight port: one thread per particle for its whole life,
- * the reference's FP64 arithmetic without FMA contraction, one atomic per deposited step.
+ * the reference's FP64 arithmetic without FMA contraction, its index formulas evaluated only near
+ * the edges of a cell, one atomic per visited cell.
  * FAST_FP32 keeps resident particle slots that refill from a work queue, pushes in FP32 with
  * two-sum compensated positions and velocities, tracks cells by comparisons, and aggregates
  * deposits in registers. FAST_FP64 is the same resident-slot engine on FP64 state and FP64
