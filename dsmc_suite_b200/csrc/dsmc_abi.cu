@@ -559,10 +559,11 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
     // absorbed flux (the reference's analytic one when none is given, thermal_model.c:130-148),
     // the initial profile from radiative balance (:172-181), and the coefficients of the
     // tridiagonal system shared by every column (:230-244, forward sweep of :80-103)
-    // one host block [|F| | initial T | c'_i | pivots] and one device block for everything
+    // one host block [|F| | initial T | c'_i | pivots | their reciprocals] and one device block for
+    // everything
     const size_t ncol = static_cast<size_t>(st.ncol), hh = static_cast<size_t>(h);
-    std::vector<double> in(2 * ncol + 2 * hh);
-    double *F = in.data(), *T_init = F + ncol, *cpv = T_init + ncol, *piv = cpv + hh;
+    std::vector<double> in(2 * ncol + 3 * hh);
+    double *F = in.data(), *T_init = F + ncol, *cpv = T_init + ncol, *piv = cpv + hh, *rcp = piv + hh;
     const double Si = CONST_SOLAR_1AU * (1.0 / tp->distance_AU) * (1.0 / tp->distance_AU);
     const double dF = Si * (1.0 - tp->albedo);
     for (int td = 0; td < ftd; td++)
@@ -587,6 +588,7 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
         piv[i] = bi - ai * cpv[i - 1];
         cpv[i] = ci / piv[i];
     }
+    for (int i = 0; i < h; i++) rcp[i] = 1.0 / piv[i];
     const size_t words = in.size() + 2 * ncol * hh + ncol;
     if (words > (size_t(1) << 30)) return fail(c, DSMC_ERR_INVALID, "thermal grid too large (%zu doubles)", words);
     if (c->scratch_bytes < words * sizeof(double)) {
@@ -605,8 +607,8 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
     if (e == cudaSuccess) e = cudaEventCreate(&ev[1]);
     if (e == cudaSuccess) e = cudaEventRecord(ev[0], c->stream);
     if (e == cudaSuccess)
-        e = dsmc::launch_thermal(st, d_in, d_in + ncol, d_in + 2 * ncol, d_in + 2 * ncol + hh, dq, ddp, dT,
-                                 c->stream);
+        e = dsmc::launch_thermal(st, d_in, d_in + ncol, d_in + 2 * ncol, d_in + 2 * ncol + hh,
+                                 d_in + 2 * ncol + 2 * hh, dq, ddp, dT, c->num_sms, c->stream);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(T_surface, dT, ncol * sizeof(double), cudaMemcpyDeviceToHost, c->stream);

@@ -39,11 +39,11 @@ struct ThermalSetup {
     double R, k_over_dr, a_last;
     double p[5], LH[5], tran_p, tran_LH, mmol;
 };
-// flux, T_init [ncol] = |F| and the initial (uniform) column temperature; cp, piv [h]; qT, dp
+// flux, T_init [ncol] = |F| and the initial (uniform) column temperature; cp, piv, rcp [h]; qT, dp
 // [h][ncol] scratch (qT ends with the final profiles); T_surface [ncol].
 cudaError_t launch_thermal(const ThermalSetup &s, const double *flux, const double *T_init,
-                           const double *cp, const double *piv, double *qT, double *dp,
-                           double *T_surface, cudaStream_t stream);
+                           const double *cp, const double *piv, const double *rcp, double *qT,
+                           double *dp, double *T_surface, int num_sms, cudaStream_t stream);
 
 // Monte Carlo shadow flux (kernel_raytrace.cu): builds the BVH of the mesh on the host, traces
 // on `stream` and copies F [nface][tt] back (synchronous). *overflows counts traversal-stack
