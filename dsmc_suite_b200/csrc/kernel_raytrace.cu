@@ -7,8 +7,15 @@
 // reference's sequence), each lifted 1e-3 along the face normal and tested for any hit along s,
 // and the face gets (1 - shadowed / Nmonte) (s . n).
 //
-// GPU design: one thread per (phase, face), consecutive threads on consecutive faces at one phase
-// (rays of a warp start close together and share the direction, so their BVH walks are coherent).
+// GPU design: one warp per (phase, face), its lanes the face's sample rays. The rays of a face start
+// in one small box and share the direction, so the warp walks the BVH once for all of them: a slab
+// test on the interval of origins (the per-ray test with each bound taken at its worst origin; the
+// float operations are monotone, so a leaf that any ray of the face enters passes) lists the
+// leaves they can enter, about 6 of a cratered sphere's. The rays then test the listed leaves
+// together, each with the test of its own: which triangles a ray is tested against, and so every
+// count, is that of a walk per ray. Such a walk took 2,820 instructions a ray at 5 of 32 lanes
+// (11.8 ms for 20,480 faces x 24 phases x 50 samples on one thread per face). The lanes enter the
+// face's random sequence at their own sample by jumping the linear congruential generator ahead.
 // The BVH is built on the host (binned surface-area heuristic, at most 4 triangles per leaf,
 // median splits below depth 40 so that every path fits the 64-entry traversal stack) and walked
 // for any hit; triangles are stored as (v0, e1, e2) float4 triples for the Moller-Trumbore test.
@@ -176,6 +183,22 @@ __device__ __forceinline__ int rand_r_dev(unsigned int *seed) {
     return result;
 }
 
+// State of rand_r's generator after `steps` steps from `seed` (x <- a x + c mod 2^32), by
+// squaring the step.
+__device__ __forceinline__ unsigned int lcg_jump(unsigned int seed, unsigned int steps) {
+    unsigned int a = 1103515245u, c = 12345u, A = 1u, C = 0u;
+    for (; steps; steps >>= 1) {
+        if (steps & 1u) {
+            A *= a;
+            C = C * a + c;
+        }
+        c *= a + 1u;
+        a *= a;
+    }
+    return A * seed + C;
+}
+constexpr unsigned int kStepsPerSample = 6;   // two rand_r calls of three steps
+
 struct ShadowArgs {
     const BvhNode *nodes;
     const float4 *tris;     // [ntri][3]: v0, e1 = v1 - v0, e2 = v2 - v0 (BVH order)
@@ -248,36 +271,127 @@ __device__ bool occluded(const ShadowArgs &a, const float o[3], const float d[3]
     return false;
 }
 
-__global__ void shadow_kernel(const ShadowArgs a) {
-    const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= static_cast<long long>(a.nface) * a.tt) return;
-    const int t = static_cast<int>(g / a.nface), nf = static_cast<int>(g % a.nface);
+// Whether any ray along d from an origin in [olo, ohi] passes slab(): the bounds of slab's interval,
+// each taken at the origin that stretches it most.
+__device__ bool slab_any(const BvhNode &n, const float olo[3], const float ohi[3], const float inv[3], float tmax) {
+    float t0 = 0.0f, t1 = tmax;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const bool up = inv[a] >= 0.0f;
+        t0 = fmaxf(t0, up ? (n.lo[a] - ohi[a]) * inv[a] : (n.hi[a] - olo[a]) * inv[a]);
+        t1 = fminf(t1, up ? (n.hi[a] - olo[a]) * inv[a] : (n.lo[a] - ohi[a]) * inv[a]);
+    }
+    return t0 <= t1;
+}
+
+constexpr int kWarps = 8;          // warps per block
+constexpr int kFacesPerWarp = 8;   // consecutive faces a warp works off
+constexpr int kLeaves = 192;       // listed leaves per warp; a face with more walks ray by ray
+
+__global__ void __launch_bounds__(32 * kWarps) shadow_kernel(const ShadowArgs a) {
+    __shared__ double sun_of_phase[3];
+    __shared__ int leaf_list[kWarps][kLeaves];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr unsigned kAll = 0xffffffffu;
     constexpr double kPi = 3.14159265358979323846;
-    const double fi = ((t + 0.5) / a.tt) * 2.0 * kPi + kPi;
-    const double sun[3] = {cos(-a.za) * sin(fi), cos(-a.za) * cos(fi), sin(-a.za)};
-    const double *fn = a.normal + 3 * nf;
-    const double c6 = sun[0] * fn[0] + sun[1] * fn[1] + sun[2] * fn[2];
-    double *out = a.F + static_cast<long long>(nf) * a.tt + t;
-    if (c6 < 0) { *out = 0.0; return; }
-    const double *A = a.spot + 3 * a.facet[3 * nf], *B = a.spot + 3 * a.facet[3 * nf + 1],
-                 *C = a.spot + 3 * a.facet[3 * nf + 2];
+    const long long groups = (a.nface + kWarps * kFacesPerWarp - 1) / (kWarps * kFacesPerWarp);
+    for (long long g = blockIdx.x; g < groups * a.tt; g += gridDim.x) {
+    const int t = static_cast<int>(g / groups);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double fi = ((t + 0.5) / a.tt) * 2.0 * kPi + kPi;
+        sun_of_phase[0] = cos(-a.za) * sin(fi);
+        sun_of_phase[1] = cos(-a.za) * cos(fi);
+        sun_of_phase[2] = sin(-a.za);
+    }
+    __syncthreads();
+    const double sun[3] = {sun_of_phase[0], sun_of_phase[1], sun_of_phase[2]};
     const float d[3] = {static_cast<float>(sun[0]), static_cast<float>(sun[1]), static_cast<float>(sun[2])};
+    const float tmax = 1e30f;
+    float inv[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) inv[k] = 1.0f / (d[k] != 0.0f ? d[k] : 1e-30f);
     const double eps = static_cast<double>(1e-3f);   // the reference's float offset, promoted
-    unsigned int seed = static_cast<unsigned int>(t * a.nface + nf + 42);
-    int shadowed = 0;
-    for (int mc = 0; mc < a.nmonte; mc++) {
-        const double r1 = sqrt(static_cast<double>(rand_r_dev(&seed)) / 2147483647.0);
-        const double r2 = static_cast<double>(rand_r_dev(&seed)) / 2147483647.0;
-        const double wa = 1.0 - r1, wb = r1 * (1.0 - r2), wc = r1 * r2;
-        float o[3];
+    int *list = leaf_list[warp];
+    const long long first = ((g % groups) * kWarps + warp) * kFacesPerWarp;
+    for (int j = 0; j < kFacesPerWarp && first + j < a.nface; j++) {
+        const int nf = static_cast<int>(first + j);
+        const double *fn = a.normal + 3 * nf;
+        const double c6 = sun[0] * fn[0] + sun[1] * fn[1] + sun[2] * fn[2];
+        double *out = a.F + static_cast<long long>(nf) * a.tt + t;
+        if (c6 < 0) {
+            if (lane == 0) *out = 0.0;
+            continue;
+        }
+        const double *A = a.spot + 3 * a.facet[3 * nf], *B = a.spot + 3 * a.facet[3 * nf + 1],
+                     *C = a.spot + 3 * a.facet[3 * nf + 2];
+        // box of the sample origins: a point of the face, lifted, rounded to float; the margin
+        // covers the rounding of the barycentric sum
+        float olo[3], ohi[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
-            const double p = A[k] * wa + B[k] * wb + C[k] * wc;
-            o[k] = static_cast<float>(p + eps * fn[k]);
+            const double lo = fmin(A[k], fmin(B[k], C[k])), hi = fmax(A[k], fmax(B[k], C[k]));
+            const double up = eps * fn[k], m = 1e-12 * (fmax(fabs(lo), fabs(hi)) + fabs(up));
+            olo[k] = __double2float_rd(lo + up - m);
+            ohi[k] = __double2float_ru(hi + up + m);
         }
-        if (occluded(a, o, d)) shadowed++;
+        // the leaves that a ray of this face can enter (every lane walks the same nodes)
+        int stack[kStack];
+        int sp = 0, n = 0, found = 0;
+        for (int it = 0; it < 2 * a.nnodes + 2; it++) {
+            const BvhNode nd = a.nodes[n];
+            bool descend = false;
+            if (slab_any(nd, olo, ohi, inv, tmax)) {
+                if (nd.count > 0) {
+                    if (found < kLeaves && lane == 0) list[found] = n;
+                    found++;
+                } else if (sp < kStack) {
+                    stack[sp++] = nd.first + 1;
+                    n = nd.first;
+                    descend = true;
+                } else if (lane == 0) {
+                    atomicAdd(a.overflow, 1);
+                }
+            }
+            if (!descend) {
+                if (sp == 0) break;
+                n = stack[--sp];
+            }
+        }
+        __syncwarp();
+        int shadowed = 0;
+        for (unsigned int base = 0; base < static_cast<unsigned int>(a.nmonte); base += 32) {
+            const unsigned int mc = base + lane;
+            const bool mine = mc < static_cast<unsigned int>(a.nmonte);
+            unsigned int seed = lcg_jump(static_cast<unsigned int>(t * a.nface + nf + 42),
+                                         kStepsPerSample * mc);
+            const double r1 = sqrt(static_cast<double>(rand_r_dev(&seed)) / 2147483647.0);
+            const double r2 = static_cast<double>(rand_r_dev(&seed)) / 2147483647.0;
+            const double wa = 1.0 - r1, wb = r1 * (1.0 - r2), wc = r1 * r2;
+            float o[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double p = A[k] * wa + B[k] * wb + C[k] * wc;
+                o[k] = static_cast<float>(p + eps * fn[k]);
+            }
+            bool hit = false;
+            if (found <= kLeaves) {
+                for (int l = 0; l < found && __any_sync(kAll, mine && !hit); l++) {
+                    const BvhNode nd = a.nodes[list[l]];
+                    if (mine && !hit && slab(nd, o, inv, tmax))
+                        for (int k = nd.first; k < nd.first + nd.count && !hit; k++)
+                            hit = hit_triangle(a.tris + 3 * k, o, d, tmax);
+                    __syncwarp();
+                }
+            } else if (mine) {
+                hit = occluded(a, o, d);
+            }
+            shadowed += __popc(__ballot_sync(kAll, mine && hit));
+        }
+        if (lane == 0) *out = (1.0 - static_cast<double>(shadowed) / a.nmonte) * c6;
+        __syncwarp();
     }
-    *out = (1.0 - static_cast<double>(shadowed) / a.nmonte) * c6;
+    }
 }
 
 }  // namespace
@@ -332,8 +446,7 @@ cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *fa
     a.za = za;
     a.F = static_cast<double *>(b.p[5]);
     a.overflow = static_cast<int *>(b.p[6]);
-    const int block = 128;
-    const long long threads = static_cast<long long>(nfc) * tt;
+    const int faces = kWarps * kFacesPerWarp;
     struct Events {
         cudaEvent_t e[2] = {nullptr, nullptr};
         ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
@@ -341,7 +454,8 @@ cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *fa
     if ((e = cudaEventCreate(&ev.e[0])) != cudaSuccess || (e = cudaEventCreate(&ev.e[1])) != cudaSuccess ||
         (e = cudaEventRecord(ev.e[0], stream)) != cudaSuccess)
         return e;
-    shadow_kernel<<<static_cast<unsigned>((threads + block - 1) / block), block, 0, stream>>>(a);
+    const long long blocks = std::min((nface + faces - 1ll) / faces * tt, 1ll << 30);
+    shadow_kernel<<<static_cast<unsigned>(blocks), 32 * kWarps, 0, stream>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ev.e[1], stream)) != cudaSuccess) return e;
     int ovf = 0;
