@@ -32,6 +32,11 @@ struct FastInst {
     int gather;              // lane-chunks a stopped lane may idle before its warp runs the events
                              // it gathered (0: no gathering), from the hop length (gather_chunks)
     double drift_abs;        // drift_tol * GM / Radii: the energy-drift guard's bound (0 = off)
+    // collision rate n * sigma per cell in the engine's precision, negative where the cell has no
+    // valid fit (the path integral grows there, no collision follows), 0 where nothing collides;
+    // built for solves of one instance (nsig_kernel), nullptr in the served queue
+    const float *nsig;
+    const double *nsigd;
     const float4 *face_f;    // FP32 icosphere tables (config model), or nullptr: FP64 descent
 };
 
@@ -294,6 +299,8 @@ private:
     FastInst *d_inst_ = nullptr;
     int ninst_cap_ = 0;
     int ninst_ = 0;
+    void *d_nsig_ = nullptr;                  // collision rates of a solve (FastInst::nsig)
+    size_t nsig_cap_ = 0;
     float *d_tab_ = nullptr;
     size_t tab_cap_ = 0;
     std::vector<float> tab_host_;             // staging of d_tab_

@@ -148,14 +148,23 @@ struct BoundsT {
 // queue) or from the block's shared memory (a solve of one instance, OneArgsT), where a cell
 // change needs a 32-bit address and no descriptor load.
 template <typename R> struct GlobalTab;
+// Collision rate n * sigma of a cell from the background density.
+__device__ __forceinline__ double background_rate(const FastInst &I, int ht, int ci) {
+    if (I.t.n_bg && I.p.runner == DSMC_RUNNER_ADVANCED && ht < I.p.collide_ht_max && ci < I.t.n_bg_len)
+        return __ldg(I.t.n_bg + ci) * I.p.cross_section;
+    return 0.0;
+}
+
 template <> struct GlobalTab<float> {
     const FastInst &I;
+    __device__ float rate(int ht, int ci) const { return static_cast<float>(background_rate(I, ht, ci)); }
     __device__ float rb2(int j) const { return __ldg(I.rb2 + j); }
     __device__ float sbs(int j) const { return __ldg(I.sbs + j); }
     __device__ float2 lon(int j) const { return __ldg(I.lonb + j); }
 };
 template <> struct GlobalTab<double> {
     const FastInst &I;
+    __device__ double rate(int ht, int ci) const { return background_rate(I, ht, ci); }
     __device__ double rb2(int j) const { return __ldg(I.rb2d + j); }
     __device__ double sbs(int j) const { return __ldg(I.sbsd + j); }
     __device__ double2 lon(int j) const { return __ldg(I.lonbd + j); }
@@ -172,6 +181,10 @@ struct SharedTab {
     __device__ static V2 *lonb() { return reinterpret_cast<V2 *>(smem_tables); }
     __device__ static R *sbsb() { return reinterpret_cast<R *>(lonb() + kRows); }
     __device__ static R *rb2b() { return sbsb() + kRows; }
+    __device__ R rate(int, int ci) const {
+        if constexpr (std::is_same<R, double>::value) return I.nsigd ? __ldg(I.nsigd + ci) : 0.0;
+        else return I.nsig ? __ldg(I.nsig + ci) : 0.0f;
+    }
     __device__ R rb2(int j) const { return rb2b()[j]; }
     __device__ R sbs(int j) const { return sbsb()[j]; }
     __device__ V2 lon(int j) const { return lonb()[j]; }
@@ -392,10 +405,7 @@ __device__ __forceinline__ void enter_cell(const T &tab, HotT<R> &h, BoundsT<R> 
     b.c0 = lo.y;
     b.s1 = hi.x;
     b.c1 = hi.y;
-    h.nsig = R(0);
-    if (I.t.n_bg && I.p.runner == DSMC_RUNNER_ADVANCED && ht < I.p.collide_ht_max &&
-        h.ci < I.t.n_bg_len)
-        h.nsig = static_cast<R>(__ldg(I.t.n_bg + h.ci) * I.p.cross_section);
+    h.nsig = tab.rate(ht, h.ci);
 }
 
 template <typename R>
@@ -491,11 +501,7 @@ __device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &
     h.cell = cell;
     h.ci = (ht * I.p.ftd + td) * I.p.ffd + fd;
     h.W = h.w0 * exp2_r<R>(-c_day_of<R>(I) * static_cast<R>(h.nday));   // re-anchor the running weight
-    if (!kNoBg && I.t.n_bg) {
-        h.nsig = R(0);
-        if (I.p.runner == DSMC_RUNNER_ADVANCED && ht < I.p.collide_ht_max && h.ci < I.t.n_bg_len)
-            h.nsig = static_cast<R>(__ldg(I.t.n_bg + h.ci) * I.p.cross_section);
-    }
+    if (!kNoBg) h.nsig = tab.rate(ht, h.ci);
     return true;
 }
 
@@ -1541,12 +1547,14 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
             if (M::kCfg || (M::kRef && taken != skip) ||
                 (M::kAny && !((k.flags & kFlagSkipFirst) && ii == 0))) {
                 bool collided = false;
-                if ((M::kAny ? (k.flags & kFlagCollide) != 0 : M::kCol) && h.nsig > R(0)) {
-                    h.pcol = fma_r(sqrt(fma_r(d[0], d[0], fma_r(d[1], d[1], d[2] * d[2]))), h.nsig, h.pcol);
-                    if (h.pcol > h.pthr) {
+                if ((M::kAny ? (k.flags & kFlagCollide) != 0 : M::kCol) &&
+                    (A::kOne ? h.nsig != R(0) : h.nsig > R(0))) {
+                    const R rate = A::kOne ? fabs(h.nsig) : h.nsig;
+                    h.pcol = fma_r(sqrt(fma_r(d[0], d[0], fma_r(d[1], d[1], d[2] * d[2]))), rate, h.pcol);
+                    if (h.pcol > h.pthr && (!A::kOne || h.nsig > R(0))) {
                         const int ht = h.cell >> 16, td = (h.cell >> 8) & 0xff, fd = h.cell & 0xff;
                         const long long pidx = (static_cast<long long>(td) * I.p.ffd + fd) * I.p.hd + ht;
-                        if (ht < k.col_ht && __ldg(I.t.cdf_valid + pidx)) {
+                        if (A::kOne || (ht < k.col_ht && __ldg(I.t.cdf_valid + pidx))) {
                             collide<kMode>(a, i, I, h, pidx);
                             collided = true;
                         }
