@@ -1461,15 +1461,23 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
         for (;;) {
         const int lim = gather ? min(n, taken + kChunk) : n;
         if constexpr (kUnroll > 1) {
-        static_assert(kMode == 1, "the sparse loop exists for the lean ballistic loop");
+        static_assert(A::kOne && !M::kAny && !M::kHist, "modes that have a sparse loop");
         gravity(q, k.GM);
         while (!event && taken < lim) {
             R d[3];
-            bool in_r = true, in_t = true, in_f = true, left = false;
+            bool in_r = true, in_t = true, in_f = true, left = false, struck = false;
             auto settle = [&]() {   // a step's photolysis and deposit, once the cell is known
-                if (fma_r(q.x, k.sx, fma_r(q.y, k.sy, q.z * k.sz)) > R(0)) {
+                const bool day = M::kRef ? ((h.cell & 0xff) < k.half_ffd)
+                                         : (fma_r(q.x, k.sx, fma_r(q.y, k.sy, q.z * k.sz)) > R(0));
+                if (day) {
                     h.nday++;
                     h.W *= k.fday;
+                }
+                if (M::kRef && taken == skip) return;
+                if (M::kCol && h.nsig != R(0)) {
+                    h.pcol = fma_r(sqrt(fma_r(d[0], d[0], fma_r(d[1], d[1], d[2] * d[2]))), fabs(h.nsig), h.pcol);
+                    struck = h.pcol > h.pthr && h.nsig > R(0);
+                    if (struck) return;
                 }
                 h.run_w += h.W;
             };
@@ -1488,6 +1496,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     break;
                 }
                 settle();
+                if (M::kCol && struck) break;
                 if (u == 0 && !whole) break;
             }
             if (left) {
@@ -1499,12 +1508,16 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
-                    q.r2 != q.r2) {
+                if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                    kMode == 1 && q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
                 }
                 settle();
+            }
+            if (M::kCol && struck) {
+                const int ht = h.cell >> 16, td = (h.cell >> 8) & 0xff, fd = h.cell & 0xff;
+                collide<kMode>(a, i, I, h, (static_cast<long long>(td) * I.p.ffd + fd) * I.p.hd + ht);
             }
         }
         } else {

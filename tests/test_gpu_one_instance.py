@@ -57,6 +57,44 @@ def test_one_instance_equals_served_kernels(N, kind, n):
             assert np.array_equal(a[key], b[key]), key
 
 
+@pytest.fixture(scope="module")
+def collisional(N):
+    """The config model's collisional problem, and the reference model's with every third cell's fit
+    invalid (a path integral then passes its threshold where no collision can follow)."""
+    from dsmc_suite_b200 import Context
+    from dsmc_suite_b200 import workloads as W
+    with Context(0) as ctx:
+        P = W.collisional_problem(ctx, "col", *BODIES["ceres"], 50, 7, W.sun_vector(0.0), 235.0, 50_000, 0)
+    c = P.collision
+    valid = c.valid.copy()
+    valid[::3] = 0
+    q = N.params_reference(N.RUNNER_ADVANCED, 36, 72)
+    q.lifetime /= 60.0
+    q.wdecay = float(np.exp(-q.dt_step / q.lifetime))
+    n_bg = np.full(q.ncell, 2e13)
+    n_bg[1::7] = -1.0
+    ref = N.CollisionInputs(n_bg, c.coef, c.box, c.total, valid, c.struct.cdf_degree)
+    return {"config": (P.params, P.surface, c), "reference": (q, N.SurfaceInputs(T_map=cold_T(N)), ref)}
+
+
+@pytest.mark.parametrize("kind,n", [("config", 33), ("config", 2001), ("config", 59_200), ("config", 59_201),
+                                    ("reference", 33), ("reference", 400)])
+def test_collisions_equal_served_kernels(N, collisional, kind, n):
+    from dsmc_suite_b200 import Context
+    p, S, col = collisional[kind]
+    res = []
+    for shape in (None, (256, 2, 3000, 2)):
+        with Context(0) as ctx:
+            if shape:
+                ctx.set_launch_shape(*shape)
+            res.append(ctx.solve(N.PATH_FAST_FP32, p, S, n, collision=col, outputs=True))
+    a, b = res
+    assert a["stats"] == b["stats"] and a["stats"]["n_collisions"] > 0
+    for key in a:
+        if key != "stats":
+            assert np.array_equal(a[key], b[key]), key
+
+
 def test_particle_without_a_position(N):
     """Two particles of one stream draw an infinite launch speed (an FP32 uniform of exactly 1),
     one at its first launch, one after 23 hops: from then on each deposits its weight into the cell
