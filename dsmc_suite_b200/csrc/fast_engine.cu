@@ -153,10 +153,10 @@ cudaError_t FastEngine::ensure_slots(int num_sms) {
     if (fp64_) {
         if (block != 128) return cudaErrorInvalidValue;   // the FP64 engine runs 128-thread blocks
         variant_ = pick_variant64(blocks_per_sm, mode_);
-        e0 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, one_kernel64(variant_, mode_, false), block, one_smem_);
+        e0 = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, one_kernel64(variant_, mode_, kAnyLanes), block, one_smem_);
     } else {
         variant_ = pick_variant(block, blocks_per_sm, mode_);
-        e0 = one_ ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, one_kernel32(variant_, mode_, false), block, one_smem_)
+        e0 = one_ ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, one_kernel32(variant_, mode_, long_hops(), kAnyLanes), block, one_smem_)
                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, served_kernel(variant_, mode_), block, 0);
     }
     if (e0 != cudaSuccess) return e0;
@@ -192,12 +192,6 @@ namespace {
 // then delays the end of the solve. 1e6 Europa-like particles in FP64 ran 25.7 ms at the full
 // limit of 16, 25.1 ms at 2 and 25.4 ms at 0; 3e5 Moon-like 8.6, 8.25 and 8.4 ms.
 constexpr int kTailGather = 2;
-
-// A launch over at most this many live particles per SM runs the sparse loop: 5e4 Moon-like
-// particles (340 per SM) take 3.9 ms against 5.4 ms in the bulk loop, 1e4 Ceres-like 2.3 ms
-// against 3.8 ms, and in the tail of larger solves 3e5 Moon-like 7.0 ms against 8.4 ms, 3e5
-// Ceres-like 10.9 against 12.5 ms (200 to 500 per SM are within 1 %).
-constexpr int kSparsePerSm = 400;
 
 // Warps per SM that a few particles are spread over: one per scheduler. More warps of fewer lanes
 // diverge less but take issue slots from one another; 1e4 Ceres-like particles ran 3.85 ms on 2
@@ -373,7 +367,7 @@ cudaError_t FastEngine::upload_one(const dsmc_params &p, const DevTables &t, lon
 }
 
 // One launch of the solve's kernel over `threads` slots (map: see drain).
-cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, const int *map, bool sparse) {
+cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, const int *map, long long lanes_per_sm) {
     const unsigned grid = static_cast<unsigned>(threads / block);   // whole blocks (see warps_for)
     auto fill = [&](auto &a, const auto &slots) {
         a.one = inst_host_;
@@ -388,11 +382,11 @@ cudaError_t FastEngine::launch_one(cudaStream_t stream, long long threads, const
     if (slot_fp64_) {
         OneArgsT<double> a{};
         fill(a, slots64_);
-        one_kernel64(variant_, mode_, sparse)<<<grid, block, one_smem_, stream>>>(a);
+        one_kernel64(variant_, mode_, lanes_per_sm)<<<grid, block, one_smem_, stream>>>(a);
     } else if (one_) {
         OneArgsT<float> a{};
         fill(a, slots_);
-        one_kernel32(variant_, mode_, sparse)<<<grid, block, one_smem_, stream>>>(a);
+        one_kernel32(variant_, mode_, long_hops(), lanes_per_sm)<<<grid, block, one_smem_, stream>>>(a);
     } else {
         launch_served(stream, mode_ <= 2 ? mode_ : 0);
     }
@@ -446,9 +440,10 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
     int *inst = slot_fp64_ ? slots64_.inst : slots_.inst;
     if ((e = cudaMemsetAsync(inst, 0xff, nslots_ * sizeof(int), stream)) != cudaSuccess) return e;
     const long long whole = start->fill_warps ? start->fill_warps * 32 : nslots_;
-    // Every launch advances each live particle by its steps or ends it, and every life is bounded
-    // by its step caps, so the queue drains. The loop still gives up (launch-timeout status) if
-    // no particle finishes for 2^28 steps, which would mean a logic error, not a long solve.
+    // Every launch advances each live particle by its steps (warp_kernel: by at least one of every
+    // kWarpUnroll) or ends it, and every life is bounded by its step caps, so the queue drains. The
+    // loop still gives up (launch-timeout status) if no particle finishes for 2^28 steps, which
+    // would mean a logic error, not a long solve.
     long long issued = 0, seen = 0, live = total, quiet = 0;
     double rate = 0.0;                    // particles taken from the queue per step
     unsigned long long next = 0, finished = 0;
@@ -465,7 +460,7 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
             threads = w * 32;
             map = d_map_ + 32;
         }
-        if ((e = launch_one(stream, threads, map, live <= static_cast<long long>(kSparsePerSm) * num_sms_)) != cudaSuccess)
+        if ((e = launch_one(stream, threads, map, (live + num_sms_ - 1) / num_sms_)) != cudaSuccess)
             return e;
         launches++;
         const int at = static_cast<int>(issued & 1);
@@ -481,7 +476,7 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
             const FastCounters &c = h_ctr_[r];
             if (c.finished >= static_cast<unsigned long long>(total)) return cudaStreamSynchronize(stream);
             rate = static_cast<double>(c.next - next) / steps_per_launch;
-            quiet = c.finished == finished ? quiet + steps_per_launch : 0;
+            quiet = c.finished == finished ? quiet + (steps_per_launch + kWarpUnroll - 1) / kWarpUnroll : 0;
             next = c.next;
             finished = c.finished;
             live = total - static_cast<long long>(finished);
@@ -498,6 +493,7 @@ cudaError_t FastEngine::run(const dsmc_params &p, const DevTables &t, bool fp64,
     if (fp64 && mode_ > 2) mode_ = 0;   // the FP64 engine has loops 0, 1 and 2
     // the kernels that take the instance with the launch exist for 128-thread blocks of the two
     // default register budgets (and FP64's two); other shapes run the served kernels
+    inst_host_.gather = gather_chunks(p);
     one_ = fp64 || pick_variant(block, blocks_per_sm, mode_) >= 4;
     one_smem_ = one_ ? one_table_bytes(p, fp64) : 0;
     cudaError_t e = ensure_slots(num_sms);

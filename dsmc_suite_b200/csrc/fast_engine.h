@@ -177,12 +177,18 @@ struct OneArgsT {
 
 template <typename R> using OneKernel = void (*)(OneArgsT<R>);
 using ServedKernel = void (*)(FastArgsT<float>);
-// Steps in a row of the sparse loop (see fast_kernel).
-constexpr int kSparseUnroll = 8;
+// Lanes per SM up to which a launch runs the loops for few particles. 5e4 Moon-like particles (340
+// per SM) take 3.5 ms in warp_kernel against 5.4 ms in the bulk loop, and the tail of 3e5 runs the
+// solve in 6.6 against 8.4 ms (200 to 500 per SM are within 1 % on five solves). Below kTinyPerSm
+// warp_kernel takes 12 steps in a row: 1e4 Ceres-like particles 2.03 ms, 2.23 at 8.
+constexpr long long kSparsePerSm = 400, kTinyPerSm = 128, kAnyLanes = 1ll << 40;
+// Steps in a row of the FP64 engine's loop for few particles, and of warp_kernel at most.
+constexpr int kSparseUnroll = 8, kWarpUnroll = 12;
 // The kernels of a solve of one instance for a register budget of blocks_per_sm blocks of 128
-// threads (FP32: 4 or 5, FP64: 3 or 4); sparse: the loop for few particles, where the mode has one.
-OneKernel<float> one_kernel32(int blocks_per_sm, int mode, bool sparse);
-OneKernel<double> one_kernel64(int blocks_per_sm, int mode, bool sparse);
+// threads (FP32: 4 or 5; FP64: 3, 4, or 5 in the lean loop) and a launch over lanes_per_sm live
+// particles per SM. long_hops: the instance's events are not gathered.
+OneKernel<float> one_kernel32(int blocks_per_sm, int mode, bool long_hops, long long lanes_per_sm);
+OneKernel<double> one_kernel64(int blocks_per_sm, int mode, long long lanes_per_sm);
 // The kernels of a queue of many instances (fast_served.cu lists the variants).
 ServedKernel served_kernel(int variant, int mode);
 
@@ -247,11 +253,12 @@ private:
     cudaError_t ensure_slots(int num_sms);
     cudaError_t upload_one(const dsmc_params &p, const DevTables &t, long long pid_begin, long long n,
                            cudaStream_t stream);
-    cudaError_t launch_one(cudaStream_t stream, long long threads, const int *map, bool sparse);
+    cudaError_t launch_one(cudaStream_t stream, long long threads, const int *map, long long lanes_per_sm);
     void launch_served(cudaStream_t stream, int mode);
     cudaError_t drain(long long total, cudaStream_t stream);
     cudaError_t capture(cudaStream_t stream, int mode, cudaGraphExec_t *out);
     long long warps_for(long long live) const;
+    bool long_hops() const { return inst_host_.gather == 0; }
     void free_graphs();
 
 public:

@@ -1172,96 +1172,105 @@ __device__ __forceinline__ int find_inst(const A &a, unsigned long long w) {
     return lo;
 }
 
-// Fill an empty slot with the next particle from the queue and launch it; particles that end
-// at their first launch are finished here and the next one is taken. Returns false when the
-// queue is empty.
+// Fills an empty slot with the next particle of the queue, at its starting point; hop_top then
+// launches it. Returns false when the queue is empty.
 template <int kMode, class A, typename R>
-__device__ __forceinline__ bool start_next(const A &a, long long i, HotT<R> &h, BoundsT<R> &b,
-                           StatAcc &st) {
-    for (;;) {
-        const unsigned long long w = grab_work(a.ctr);
-        if (w >= a.ctr->total) return false;
-        const int ii = find_inst(a, w);
-        const FastInst &I = a.inst(ii);
-        const dsmc_params &p = I.p;
-        if (ii != st.inst) {
-            flush_stats_lane(a, st);
-            st.inst = ii;
+__device__ __forceinline__ bool take_next(const A &a, long long i, HotT<R> &h, StatAcc &st, R &thi,
+                                          R &fi, R &local_T) {
+    local_T = R(0);
+    const unsigned long long w = grab_work(a.ctr);
+    if (w >= a.ctr->total) return false;
+    const int ii = find_inst(a, w);
+    const FastInst &I = a.inst(ii);
+    const dsmc_params &p = I.p;
+    if (ii != st.inst) {
+        flush_stats_lane(a, st);
+        st.inst = ii;
+    }
+    const unsigned pid = static_cast<unsigned>(I.pid_begin + static_cast<long long>(w - I.work_base));
+    h.inst = ii;
+    Philox rng;
+    rng.init(p.seed, p.instance, pid);
+    philox_next<Mode<kMode>::kRoll>(rng);
+    h.w0 = R(1);
+    h.nday = 0;
+    h.steps = 0;
+    h.hop = 0;
+    h.pcol = R(0);
+    h.ci = -1;
+    h.run_w = R(0);
+    h.hist_key = -1;
+    h.hist_cnt = 0;
+    const double zero[3] = {0.0, 0.0, 0.0};
+    set_vel(h, zero);
+    double col_p = 0.0;
+    double s[3];
+    if (Mode<kMode>::ref(p)) {
+        const bool adv = p.runner == DSMC_RUNNER_ADVANCED;
+        if (adv) col_p = rng.raw(0) / kTwo32;
+        const int o = adv ? 1 : 0;
+        const double th = rng.raw(o) / kTwo32 * kPi - kPi / 2.0;
+        const double ph = rng.raw(o + 1) / kTwo32 * 2.0 * kPi;
+        s[0] = p.Radii * cos(th) * sin(ph);
+        s[1] = p.Radii * cos(th) * cos(ph);
+        s[2] = p.Radii * sin(th);
+        thi = static_cast<R>(th);
+        fi = static_cast<R>(ph);
+        int td, fd;
+        ref_index(thi, fi, p.ftd, p.ffd, td, fd);
+        local_T = static_cast<R>(I.t.T_map[td * p.ffd + fd]);
+    } else {
+        const int f = pick_face(I.t, rng.raw(0) / kTwo32);
+        a.s.face[i] = f;
+        double u1 = rng.raw(1) / kTwo32, u2 = rng.raw(2) / kTwo32;
+        col_p = rng.raw(3) / kTwo32;
+        if (u1 + u2 > 1.0) { u1 = 1.0 - u1; u2 = 1.0 - u2; }
+        const double *fv = I.t.face_verts + 9 * f;
+        double q[3];
+        for (int k = 0; k < 3; k++) q[k] = fv[k] + u1 * (fv[3 + k] - fv[k]) + u2 * (fv[6 + k] - fv[k]);
+        // |q|^-1 from the FP32 estimate and one Newton step in FP64 (relative error ~1e-14)
+        const double q2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
+        double iq = rsqrtf(static_cast<float>(q2));
+        iq = iq * (1.5 - 0.5 * q2 * iq * iq);
+        for (int k = 0; k < 3; k++) s[k] = q[k] * (p.Radii * iq);
+        local_T = static_cast<R>(I.t.face_T[f]);
+        thi = fi = R(0);   // the config model's launch does not use the angles
+    }
+    a.s.pid[i] = pid;
+    a.s.evt[i] = rng.event;
+    a.s.ncol[i] = 0;
+    a.s.rest[i] = 0.0f;
+    if (p.runner != DSMC_RUNNER_ADVANCED) {
+        h.pthr = R(0);
+    } else {
+        if constexpr (is_f64<R>()) h.pthr = -log1p(-col_p);
+        else h.pthr = -log1pf(-static_cast<float>(col_p));
+    }
+    set_pos(h, s);
+    const long long slot = static_cast<long long>(pid) - I.t.out_base;
+    if (I.t.ttime && slot >= 0 && slot < I.t.out_cap) {
+        if (p.model != DSMC_MODEL_REFERENCE) angles_of(h, thi, fi);
+        I.t.ttime[slot] = thi;
+        if (p.runner == DSMC_RUNNER_ADVANCED || p.model != DSMC_MODEL_REFERENCE) {
+            I.t.ttime[5 * I.t.out_cap + slot] = fi;
+            I.t.ttime[6 * I.t.out_cap + slot] = local_T;
         }
-        const unsigned pid = static_cast<unsigned>(I.pid_begin + static_cast<long long>(w - I.work_base));
-        h.inst = ii;
-        Philox rng;
-        rng.init(p.seed, p.instance, pid);
-        philox_next<Mode<kMode>::kRoll>(rng);
-        h.w0 = R(1);
-        h.nday = 0;
-        h.steps = 0;
-        h.hop = 0;
-        h.pcol = R(0);
-        h.ci = -1;
-        h.run_w = R(0);
-        h.hist_key = -1;
-        h.hist_cnt = 0;
-        const double zero[3] = {0.0, 0.0, 0.0};
-        set_vel(h, zero);
-        R thi, fi, local_T = R(0);
-        double col_p = 0.0;
-        double s[3];
-        if (Mode<kMode>::ref(p)) {
-            const bool adv = p.runner == DSMC_RUNNER_ADVANCED;
-            if (adv) col_p = rng.raw(0) / kTwo32;
-            const int o = adv ? 1 : 0;
-            const double th = rng.raw(o) / kTwo32 * kPi - kPi / 2.0;
-            const double ph = rng.raw(o + 1) / kTwo32 * 2.0 * kPi;
-            s[0] = p.Radii * cos(th) * sin(ph);
-            s[1] = p.Radii * cos(th) * cos(ph);
-            s[2] = p.Radii * sin(th);
-            thi = static_cast<R>(th);
-            fi = static_cast<R>(ph);
-            int td, fd;
-            ref_index(thi, fi, p.ftd, p.ffd, td, fd);
-            local_T = static_cast<R>(I.t.T_map[td * p.ffd + fd]);
-        } else {
-            const int f = pick_face(I.t, rng.raw(0) / kTwo32);
-            a.s.face[i] = f;
-            double u1 = rng.raw(1) / kTwo32, u2 = rng.raw(2) / kTwo32;
-            col_p = rng.raw(3) / kTwo32;
-            if (u1 + u2 > 1.0) { u1 = 1.0 - u1; u2 = 1.0 - u2; }
-            const double *fv = I.t.face_verts + 9 * f;
-            double q[3];
-            for (int k = 0; k < 3; k++) q[k] = fv[k] + u1 * (fv[3 + k] - fv[k]) + u2 * (fv[6 + k] - fv[k]);
-            // |q|^-1 from the FP32 estimate and one Newton step in FP64 (relative error ~1e-14)
-            const double q2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
-            double iq = rsqrtf(static_cast<float>(q2));
-            iq = iq * (1.5 - 0.5 * q2 * iq * iq);
-            for (int k = 0; k < 3; k++) s[k] = q[k] * (p.Radii * iq);
-            local_T = static_cast<R>(I.t.face_T[f]);
-            thi = fi = R(0);   // the config model's launch does not use the angles
-        }
-        a.s.pid[i] = pid;
-        a.s.evt[i] = rng.event;
-        a.s.ncol[i] = 0;
-        a.s.rest[i] = 0.0f;
-        if (p.runner != DSMC_RUNNER_ADVANCED) {
-            h.pthr = R(0);
-        } else {
-            if constexpr (is_f64<R>()) h.pthr = -log1p(-col_p);
-            else h.pthr = -log1pf(-static_cast<float>(col_p));
-        }
-        set_pos(h, s);
-        const long long slot = static_cast<long long>(pid) - I.t.out_base;
-        if (I.t.ttime && slot >= 0 && slot < I.t.out_cap) {
-            if (p.model != DSMC_MODEL_REFERENCE) angles_of(h, thi, fi);
-            I.t.ttime[slot] = thi;
-            if (p.runner == DSMC_RUNNER_ADVANCED || p.model != DSMC_MODEL_REFERENCE) {
-                I.t.ttime[5 * I.t.out_cap + slot] = fi;
-                I.t.ttime[6 * I.t.out_cap + slot] = local_T;
-            }
-        }
+    }
+    return true;
+}
+
+// Fills an empty slot with the next particle and launches it; particles that end at their first
+// launch are finished here and the next one is taken.
+template <int kMode, class A, typename R>
+__device__ __forceinline__ bool start_next(const A &a, long long i, HotT<R> &h, BoundsT<R> &b, StatAcc &st) {
+    R thi, fi, local_T;
+    while (take_next<kMode>(a, i, h, st, thi, fi, local_T)) {
+        const FastInst &I = a.inst(h.inst);
         const int fate = hop_top<kMode>(a, i, I, h, b, st, thi, fi, local_T, true);
         if (fate == 0) return true;
         finish(a, i, I, h, st, fate);
     }
+    return false;
 }
 
 // Position of the particle being pushed, with |s|^2 and the acceleration there (FP32: the velocity
@@ -1461,23 +1470,15 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
         for (;;) {
         const int lim = gather ? min(n, taken + kChunk) : n;
         if constexpr (kUnroll > 1) {
-        static_assert(A::kOne && !M::kAny && !M::kHist, "modes that have a sparse loop");
+        static_assert(kMode == 1, "the sparse loop exists for the lean ballistic loop");
         gravity(q, k.GM);
         while (!event && taken < lim) {
             R d[3];
-            bool in_r = true, in_t = true, in_f = true, left = false, struck = false;
+            bool in_r = true, in_t = true, in_f = true, left = false;
             auto settle = [&]() {   // a step's photolysis and deposit, once the cell is known
-                const bool day = M::kRef ? ((h.cell & 0xff) < k.half_ffd)
-                                         : (fma_r(q.x, k.sx, fma_r(q.y, k.sy, q.z * k.sz)) > R(0));
-                if (day) {
+                if (fma_r(q.x, k.sx, fma_r(q.y, k.sy, q.z * k.sz)) > R(0)) {
                     h.nday++;
                     h.W *= k.fday;
-                }
-                if (M::kRef && taken == skip) return;
-                if (M::kCol && h.nsig != R(0)) {
-                    h.pcol = fma_r(sqrt(fma_r(d[0], d[0], fma_r(d[1], d[1], d[2] * d[2]))), fabs(h.nsig), h.pcol);
-                    struck = h.pcol > h.pthr && h.nsig > R(0);
-                    if (struck) return;
                 }
                 h.run_w += h.W;
             };
@@ -1496,7 +1497,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     break;
                 }
                 settle();
-                if (M::kCol && struck) break;
                 if (u == 0 && !whole) break;
             }
             if (left) {
@@ -1508,16 +1508,12 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
-                    kMode == 1 && q.r2 != q.r2) {
+                if (!move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                    q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
                 }
                 settle();
-            }
-            if (M::kCol && struck) {
-                const int ht = h.cell >> 16, td = (h.cell >> 8) & 0xff, fd = h.cell & 0xff;
-                collide<kMode>(a, i, I, h, (static_cast<long long>(td) * I.p.ffd + fd) * I.p.hd + ht);
             }
         }
         } else {
@@ -1624,6 +1620,183 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
     const unsigned fin = st.finished;
     flush_stats(a, st);
     const unsigned wfin = __reduce_add_sync(0xffffffffu, fin);
+    if ((threadIdx.x & 31) == 0 && wfin) atomicAdd(&a.ctr->finished, static_cast<unsigned long long>(wfin));
+}
+
+enum Event { kEvNone = 0, kEvLanded, kEvEscaped, kEvCap, kEvEmpty, kEvResume };
+
+// The step loop of fast_kernel kept in step warp by warp: all lanes take up to kUnroll steps in a
+// row without a branch back, the next step's reciprocal square root beside this step's cell tests;
+// a lane that leaves its cell (or collides) stops there, and the lanes that did take the slow path
+// together; events (landing, escape, cap, an empty slot) run at one place, for all lanes that have
+// one, once the lanes that wait have idled `limit` iterations in all. Against fast_kernel, whose
+// lanes take every cell change as it comes, a change costs its lane the rest of the iteration, but
+// the change's code runs once per iteration and not once per step (a warp of long hops changes a
+// cell on half of its steps), the branches per step halve, and the event code exists once.
+// A launch runs a.K / kUnroll iterations, so a lane takes at most a.K steps.
+// Measured at kUnroll 8: 1e7 Ceres-like particles 280.4 ms against 291.5 ms, 3e5 of the reference
+// model 72 against 103 ms; 4 and 12 steps in a row ran the former in 307 and 297 ms. Few particles,
+// whose warps have nothing to hide a branch behind: 512 Ceres-like 1.60 ms at 12 steps in a row,
+// 1.77 at 8, 3.4 in fast_kernel; 500 of the reference model with collisions 42.9 ms at 12, 46.7 at
+// 8, 59.4 in fast_kernel. It loses where events are frequent for the steps they wait: 3e6 Moon-like
+// particles 44.7 against 42.5 ms, with histograms 50 against 45 ms, collisions 62 against 49 ms.
+template <int kMaxThreads, int kMinBlocks, int kMode, int kUnroll>
+__global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __grid_constant__ OneArgsT<float> a) {
+    using A = OneArgsT<float>;
+    using R = float;
+    using M = Mode<kMode>;
+    using Tab = TabOf<A, R>;
+    constexpr unsigned kAll = 0xffffffffu;
+    SharedTab<R>::fill(a.one);
+    const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long long i = a.slot(t);
+    HotT<R> h;
+    if (i >= 0) load_hot(a.s, i, a.nslots, h);
+    else h.inst = -1;
+    StatAcc st;
+    st.inst = h.inst;
+    const FastInst &I = a.one;
+    const StepConst<R> &k = a.k;
+    BoundsT<R> b;
+    bool flying = h.inst >= 0;
+    int event = flying ? kEvResume : kEvNone;
+
+    if (flying) {
+        // reload the cached bounds of the saved cell without flushing its pending deposits
+        const int ci = h.ci;
+        const R run_w = h.run_w;
+        h.ci = -1;
+        enter_cell(Tab{I}, h, b, h.cell);
+        h.ci = ci;
+        h.run_w = run_w;
+    } else if (i >= 0) {
+        // a queue of fewer particles than slots starts on the lanes that fill_warps chose
+        const long long warps = a.ctr->fill_warps;
+        if (warps == 0 || ((t >> 5) < warps && (t & 31) * warps + (t >> 5) < static_cast<long long>(a.ctr->total)))
+            event = kEvEmpty;
+    }
+    PosT<R> q;
+    int n = 0, taken = 0, skip = 0, idle = 0;
+    const int limit = a.gather * kChunk / kUnroll;   // lane-chunks of kChunk steps in lane-iterations
+
+    const bool work = __any_sync(kAll, event != kEvNone);
+    const int iters = a.K / kUnroll > 0 ? a.K / kUnroll : 1;
+    for (int it = 0; work; it++) {
+        const bool last = it >= iters;
+        const unsigned ev = __ballot_sync(kAll, event != kEvNone);
+        if (ev || last) {
+            idle += __popc(ev);
+            const unsigned fly = __ballot_sync(kAll, flying && !event);
+            if (idle >= limit || !fly || last) {
+                idle = 0;
+                if (event) {
+                    int fate = event == kEvResume ? 0 : -1;
+                    R thi = R(0), fi = R(0), local_T = R(0);
+                    if (event == kEvLanded || event == kEvEscaped || event == kEvCap) {
+                        st.steps += taken;
+                        h.steps += taken;
+                        taken = 0;
+                        drift_check(a, i, I, h, st);
+                        fate = event == kEvEscaped ? DSMC_FATE_ESCAPED
+                             : event == kEvCap ? DSMC_FATE_STEP_CAP : land<kMode>(a, i, I, h, thi, fi, local_T);
+                    }
+                    if (event != kEvResume) {
+                        bool first = false;
+                        for (;;) {
+                            if (fate) {
+                                if (fate > 0) finish(a, i, I, h, st, fate);
+                                flying = take_next<kMode>(a, i, h, st, thi, fi, local_T);
+                                if (!flying) break;
+                                first = true;
+                            }
+                            fate = hop_top<kMode>(a, i, I, h, b, st, thi, fi, local_T, first);
+                            if (!fate) break;
+                        }
+                    }
+                    event = 0;
+                    if (flying) {
+                        start_pos(h, q);
+                        gravity(q, k.GM);
+                        n = 0x7fffffff;
+                        if (!M::kRef) n = min(n, k.life_cap - h.steps);
+                        if (!M::kCfg) n = min(n, k.hop_cap - h.hop);
+                        // the step that the skip-first rule leaves without a deposit
+                        skip = !M::kCfg && (k.flags & kFlagSkipFirst) && h.hop == 0 ? 1 : 0;
+                        taken = 0;
+                    }
+                }
+                __syncwarp();
+            }
+            if (last || !__any_sync(kAll, flying)) break;
+        }
+        R d[3];
+        bool in_r = true, in_t = true, in_f = true;
+        bool left = false, struck = false;
+        auto settle = [&]() {   // a step's photolysis and deposit, once the cell is known
+            const bool day = M::kRef ? ((h.cell & 0xff) < k.half_ffd)
+                                     : (fma_r(q.x, k.sx, fma_r(q.y, k.sy, q.z * k.sz)) > R(0));
+            if (day) {
+                h.nday++;
+                h.W *= k.fday;
+            }
+            if (M::kRef && taken == skip) return;
+            if (M::kCol && h.nsig != R(0)) {
+                h.pcol = fma_r(sqrt(fma_r(d[0], d[0], fma_r(d[1], d[1], d[2] * d[2]))), fabs(h.nsig), h.pcol);
+                struck = h.pcol > h.pthr && h.nsig > R(0);
+                if (struck) return;
+            }
+            h.run_w += h.W;
+        };
+        if (flying && !event) {
+            const bool whole = n - taken >= kUnroll;
+#pragma unroll
+            for (int u = 0; u < kUnroll; u++) {
+                verlet_step(h, q, k.dt, k.c1, k.c2, d);
+                gravity(q, k.GM);
+                taken++;
+                const R zz = q.z * fabs(q.z);
+                in_r = (q.r2 > b.r2lo) & (q.r2 <= b.r2hi);
+                in_t = (zz > q.r2 * b.zlo) & (zz <= q.r2 * b.zhi);
+                in_f = (q.x * b.c0 - q.y * b.s0 > R(0)) & (q.x * b.c1 - q.y * b.s1 <= R(0));
+                if (!(in_r & in_t & in_f)) {
+                    left = true;
+                    break;
+                }
+                settle();
+                if (M::kCol && struck) break;
+                if (u == 0 && !whole) break;
+            }
+        }
+        __syncwarp();
+        if (left) {
+            if (q.r2 <= k.rl2) {
+                event = kEvLanded;
+            } else if (q.r2 >= k.re2) {
+                event = kEvEscaped;
+            } else if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                       kMode == 1 && q.r2 != q.r2) {
+                taken = drift_nowhere(h, taken, n);
+            } else {
+                settle();
+            }
+        }
+        if (M::kCol && struck) {
+            const int ht = h.cell >> 16, td = (h.cell >> 8) & 0xff, fd = h.cell & 0xff;
+            collide<kMode>(a, i, I, h, (static_cast<long long>(td) * I.p.ffd + fd) * I.p.hd + ht);
+        }
+        if (flying && !event && taken >= n)
+            event = !M::kRef && h.steps + taken >= k.life_cap ? kEvCap : kEvLanded;
+    }
+    if (flying) {
+        st.steps += taken;
+        h.steps += taken;
+        if (!M::kCfg) h.hop += taken;
+    }
+    if (i >= 0) store_hot(a.s, i, a.nslots, h);
+    // statistics of this launch, per instance; the finished count also drives the host loop
+    const unsigned fin = st.finished;
+    flush_stats(a, st);
+    const unsigned wfin = __reduce_add_sync(kAll, fin);
     if ((threadIdx.x & 31) == 0 && wfin) atomicAdd(&a.ctr->finished, static_cast<unsigned long long>(wfin));
 }
 

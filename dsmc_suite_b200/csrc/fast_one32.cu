@@ -5,15 +5,14 @@
 namespace dsmc {
 namespace {
 
-template <int kB, int kMode, int kUnroll = 1>
-constexpr OneKernel<float> one() { return fast_kernel<128, kB, kMode, kUnroll, OneArgsT<float>, float>; }
+template <int kB, int kMode>
+constexpr OneKernel<float> one() { return fast_kernel<128, kB, kMode, 1, OneArgsT<float>, float>; }
 
 template <int kB>
 OneKernel<float> by_mode(int mode) {
     switch (mode) {
         case 1: return one<kB, 1>();
         case 2: return one<kB, 2>();
-        case 3: return one<kB, 3>();
         case 4: return one<kB, 4>();
         case 5: return one<kB, 5>();
         default: return one<kB, 0>();
@@ -57,13 +56,18 @@ __global__ void push_fp32_kernel(const dsmc_params p, long long n, int nsteps, d
 
 }  // namespace
 
-OneKernel<float> one_kernel32(int blocks_per_sm, int mode, bool sparse) {
-    // 1e4 particles of the collisional config model run 4.75 ms in the sparse loop against 5.58 ms,
-    // 500 of the reference model with collisions 45.9 against 59.4 ms; without collisions the
-    // reference model's time is its landings (24.6 against 24.7 ms), and it keeps one loop
-    if (sparse && mode == 1) return one<4, 1, kSparseUnroll>();
-    if (sparse && mode == 2) return one<4, 2, kSparseUnroll>();
-    if (sparse && mode == 5) return one<4, 5, kSparseUnroll>();
+// Which loop (see fast_kernel and warp_kernel for both sides' times): the warp's step loop for few
+// lanes per SM, in every mode that has one, and for the bulk where hops are long (ballistic config
+// model) or events are most of the work (reference model); elsewhere the free-running lanes.
+OneKernel<float> one_kernel32(int blocks_per_sm, int mode, bool long_hops, long long lanes_per_sm) {
+    if (lanes_per_sm <= kSparsePerSm) {
+        if (mode == 1) return lanes_per_sm <= kTinyPerSm ? warp_kernel<128, 4, 1, 12> : warp_kernel<128, 4, 1, 8>;
+        if (mode == 2) return warp_kernel<128, 4, 2, 12>;
+        if (mode == 3) return warp_kernel<128, 4, 3, 8>;
+        if (mode == 5) return warp_kernel<128, 4, 5, 12>;
+    }
+    if (mode == 3) return blocks_per_sm == 5 ? warp_kernel<128, 5, 3, 8> : warp_kernel<128, 4, 3, 8>;
+    if (mode == 1 && long_hops) return blocks_per_sm == 5 ? warp_kernel<128, 5, 1, 8> : warp_kernel<128, 4, 1, 8>;
     return blocks_per_sm == 5 ? by_mode<5>(mode) : by_mode<4>(mode);
 }
 

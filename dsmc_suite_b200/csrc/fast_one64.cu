@@ -14,8 +14,8 @@ OneKernel<double> by_mode(int mode) {
 
 }  // namespace
 
-OneKernel<double> one_kernel64(int blocks_per_sm, int mode, bool sparse) {
-    if (sparse && mode == 1) return one<4, 1, kSparseUnroll>();
+OneKernel<double> one_kernel64(int blocks_per_sm, int mode, long long lanes_per_sm) {
+    if (lanes_per_sm <= kSparsePerSm && mode == 1) return one<4, 1, kSparseUnroll>();
     if (blocks_per_sm == 5) return one<5, 1>();   // the lean loop only
     return blocks_per_sm == 3 ? by_mode<3>(mode) : by_mode<4>(mode);
 }

@@ -1,8 +1,8 @@
 """A solve of one instance against the kernels of the served queue (needs a B200).
 
 A solve in the default launch shape runs loops that take the instance with the launch, start few
-particles on a lane spread, switch to the sparse loop below a particle count and pack the live
-slots once the queue is empty; a 256-thread shape runs the general loops of the served queue over
+particles on a lane spread, switch to the loops for few particles below a particle count and pack
+the live slots once the queue is empty; a 256-thread shape runs the general loops of the served queue over
 descriptors in device memory. A particle's trajectory, random stream and deposits are functions of
 its id alone, so both give the same grids, rows and counters bit for bit."""
 from __future__ import annotations
@@ -15,9 +15,9 @@ from conftest import cold_T
 pytestmark = pytest.mark.gpu
 
 BODIES = {"ceres": (470e3, 6.26e10), "moon": (1737e3, 4.90e12)}
-# edges of a warp, of one warp per scheduler, of the sparse loop's range and of the slots (640 per
-# SM), on a GPU of 148 SMs
-SIZES = [1, 33, 593, 59_200, 59_201, 94_719, 94_721, 200_003]
+# edges of a warp, of one warp per scheduler, of the ranges of the loops for few particles and of the
+# slots (640 per SM), on a GPU of 148 SMs
+SIZES = [1, 33, 593, 18_944, 18_945, 59_200, 59_201, 94_719, 94_721, 200_003]
 
 
 def _problem(N, kind):
