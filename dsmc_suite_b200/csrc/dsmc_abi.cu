@@ -36,7 +36,7 @@ struct dsmc_ctx {
     dsmc::FastEngine *fast = nullptr;
     long long last_launches = 0;
     double last_kernel_ms = 0.0;     // device time of the last thermal / shadow-flux kernel
-    void *scratch = nullptr;          // grow-only device scratch of the thermal solve
+    void *scratch = nullptr;          // device scratch of the synchronous calls (need_scratch)
     size_t scratch_bytes = 0;
     char err[512] = {0};
 };
@@ -84,6 +84,41 @@ void free_outputs(dsmc_ctx *c) {
     c->t.out_cap = 0;
     c->t.out_base = 0;
 }
+
+// Device scratch of at least `bytes` bytes, kept by the context up to kScratchKept bytes (a call
+// that needed more gives it back: ScratchUse). Its users are synchronous calls on one context.
+constexpr size_t kScratchKept = size_t(256) << 20;
+
+int need_scratch(dsmc_ctx *c, size_t bytes) {
+    if (c->scratch_bytes >= bytes) return DSMC_OK;
+    DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (c->scratch) cudaFree(c->scratch);
+    c->scratch = nullptr;
+    c->scratch_bytes = 0;
+    DSMC_CUDA_TRY(c, cudaMalloc(&c->scratch, bytes));
+    c->scratch_bytes = bytes;
+    return DSMC_OK;
+}
+
+// Parts of the scratch, each on a 256-byte boundary: sizes first (part), then addresses (at).
+struct ScratchUse {
+    dsmc_ctx *c;
+    std::vector<size_t> start;
+    size_t total = 0;
+    explicit ScratchUse(dsmc_ctx *ctx) : c(ctx) {}
+    ~ScratchUse() {
+        if (c->scratch_bytes <= kScratchKept) return;
+        cudaStreamSynchronize(c->stream);
+        cudaFree(c->scratch);
+        c->scratch = nullptr;
+        c->scratch_bytes = 0;
+    }
+    void part(size_t bytes) {
+        start.push_back(total);
+        total += (bytes + 255) & ~size_t(255);
+    }
+    void *at(size_t k) const { return static_cast<char *>(c->scratch) + start[k]; }
+};
 
 }  // namespace
 
@@ -164,8 +199,10 @@ int dsmc_setup(dsmc_ctx *c, const dsmc_params *p, const dsmc_surface *s,
     int rc = dsmc::problem_check(p, s, col, c->err, sizeof c->err);
     if (rc != DSMC_OK) return rc;
     if ((rc = set_device(c)) != DSMC_OK) return rc;
-    DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    free_tables(c);
+    // nothing may still read the tables that the new problem takes over, on any stream the context
+    // was given
+    DSMC_CUDA_TRY(c, cudaDeviceSynchronize());
+    c->ready = false;
     rc = dsmc::problem_build(c->prob, p, s, col, c->stats, c->stream, false, c->err, sizeof c->err);
     if (rc != DSMC_OK) {
         free_tables(c);
@@ -194,6 +231,13 @@ int dsmc_enable_particle_outputs(dsmc_ctx *c, int64_t n) {
     int rc = set_device(c);
     if (rc != DSMC_OK) return rc;
     DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    if (n > 0 && n == c->t.out_cap) {   // the same rows again: cleared, as new ones are
+        c->t.out_base = 0;
+        DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[0], 0, static_cast<size_t>(n) * 9 * sizeof(double), c->stream));
+        DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[1], 0, static_cast<size_t>(n) * sizeof(int), c->stream));
+        DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[2], 0, static_cast<size_t>(n) * sizeof(long long), c->stream));
+        return DSMC_OK;
+    }
     free_outputs(c);
     if (n == 0) return DSMC_OK;
     DSMC_CUDA_TRY(c, cudaMalloc(&c->outputs[0], static_cast<size_t>(n) * 9 * sizeof(double)));
@@ -413,24 +457,24 @@ int dsmc_horizon_device(dsmc_ctx *c, uint64_t **dev_ptr, int64_t *ncell) {
 
 namespace {
 
-// Temporary device buffers of one fit call, freed on every exit path.
+// Device buffers of one fit call: input, counts, coefficients, boxes, totals, validity.
 struct FitBuffers {
+    ScratchUse use;
     void *p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    ~FitBuffers() { for (void *q : p) if (q) cudaFree(q); }
+    explicit FitBuffers(dsmc_ctx *c) : use(c) {}
 };
 
 int fit_common(dsmc_ctx *c, FitBuffers &b, int64_t ncell, size_t in_bytes, const void *in_host,
                const int32_t *counts) {
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[0], in_bytes));
+    const size_t sizes[6] = {in_bytes, counts ? ncell * sizeof(int) : 0, ncell * DSMC_CDF_STRIDE * sizeof(double),
+                             ncell * 4 * sizeof(double), ncell * sizeof(double), ncell * sizeof(int)};
+    for (size_t n : sizes) b.use.part(n);
+    const int rc = need_scratch(c, b.use.total);
+    if (rc != DSMC_OK) return rc;
+    for (int k = 0; k < 6; k++) b.p[k] = b.use.at(k);
     DSMC_CUDA_TRY(c, cudaMemcpyAsync(b.p[0], in_host, in_bytes, cudaMemcpyHostToDevice, c->stream));
-    if (counts) {
-        DSMC_CUDA_TRY(c, cudaMalloc(&b.p[1], ncell * sizeof(int)));
+    if (counts)
         DSMC_CUDA_TRY(c, cudaMemcpyAsync(b.p[1], counts, ncell * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    }
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[2], ncell * DSMC_CDF_STRIDE * sizeof(double)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[3], ncell * 4 * sizeof(double)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[4], ncell * sizeof(double)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[5], ncell * sizeof(int)));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(b.p[3], 0, ncell * 4 * sizeof(double), c->stream));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(b.p[4], 0, ncell * sizeof(double), c->stream));
     return DSMC_OK;
@@ -457,7 +501,7 @@ int dsmc_fit_cdf_samples_host(dsmc_ctx *c, int64_t ncell, int max_per_cell, cons
         return fail(c, DSMC_ERR_INVALID, "fit: bad sizes");
     int rc = set_device(c);
     if (rc != DSMC_OK) return rc;
-    FitBuffers b;
+    FitBuffers b(c);
     if ((rc = fit_common(c, b, ncell, ncell * max_per_cell * sizeof(double), speeds, counts)) != DSMC_OK)
         return rc;
     DSMC_CUDA_TRY(c, dsmc::launch_fit_samples(static_cast<int>(ncell), max_per_cell,
@@ -478,7 +522,7 @@ int dsmc_fit_cdf_hist_host(dsmc_ctx *c, int64_t ncell, int nbins, double bin_wid
         return fail(c, DSMC_ERR_INVALID, "fit: bad sizes");
     int rc = set_device(c);
     if (rc != DSMC_OK) return rc;
-    FitBuffers b;
+    FitBuffers b(c);
     if ((rc = fit_common(c, b, ncell, ncell * nbins * sizeof(uint64_t), hist, nullptr)) != DSMC_OK)
         return rc;
     DSMC_CUDA_TRY(c, dsmc::launch_fit_hist(static_cast<int>(ncell), nbins, bin_width,
@@ -497,15 +541,11 @@ int dsmc_push_host(dsmc_ctx *c, int path, int64_t n, int nsteps, double *pos, do
         return fail(c, DSMC_ERR_INVALID, "unknown path %d", path);
     int rc = set_device(c);
     if (rc != DSMC_OK || n == 0) return rc;
-    struct Bufs {
-        void *p[4] = {nullptr, nullptr, nullptr, nullptr};
-        ~Bufs() { for (void *q : p) if (q) cudaFree(q); }
-    } b;
     const size_t vb = static_cast<size_t>(n) * 3 * sizeof(double);
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[0], vb));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[1], vb));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[2], n * sizeof(int)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[3], n * sizeof(int)));
+    ScratchUse use(c);
+    for (size_t bytes : {vb, vb, n * sizeof(int), n * sizeof(int)}) use.part(bytes);
+    if ((rc = need_scratch(c, use.total)) != DSMC_OK) return rc;
+    struct { void *p[4]; } b = {{use.at(0), use.at(1), use.at(2), use.at(3)}};
     DSMC_CUDA_TRY(c, cudaMemcpyAsync(b.p[0], pos, vb, cudaMemcpyHostToDevice, c->stream));
     DSMC_CUDA_TRY(c, cudaMemcpyAsync(b.p[1], vel, vb, cudaMemcpyHostToDevice, c->stream));
     double *dp = static_cast<double *>(b.p[0]), *dv = static_cast<double *>(b.p[1]);
@@ -591,14 +631,8 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
     for (int i = 0; i < h; i++) rcp[i] = 1.0 / piv[i];
     const size_t words = in.size() + 2 * ncol * hh + ncol;
     if (words > (size_t(1) << 30)) return fail(c, DSMC_ERR_INVALID, "thermal grid too large (%zu doubles)", words);
-    if (c->scratch_bytes < words * sizeof(double)) {
-        DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        if (c->scratch) cudaFree(c->scratch);
-        c->scratch = nullptr;
-        c->scratch_bytes = 0;
-        DSMC_CUDA_TRY(c, cudaMalloc(&c->scratch, words * sizeof(double)));
-        c->scratch_bytes = words * sizeof(double);
-    }
+    ScratchUse use(c);
+    if ((rc = need_scratch(c, words * sizeof(double))) != DSMC_OK) return rc;
     double *d_in = static_cast<double *>(c->scratch);
     double *dq = d_in + in.size(), *ddp = dq + ncol * hh, *dT = ddp + ncol * hh;
     cudaError_t e = cudaMemcpyAsync(d_in, in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
@@ -639,8 +673,12 @@ int dsmc_shadow_flux_host(dsmc_ctx *c, int npoint, const double *spot, int nface
     int rc = set_device(c);
     if (rc != DSMC_OK) return rc;
     long long overflows = 0;
-    DSMC_CUDA_TRY(c, dsmc::shadow_flux(npoint, spot, nface, facet, face_normal, za, tt, nmonte, F,
-                                       c->stream, &overflows, &c->last_kernel_ms));
+    ScratchUse use(c);
+    auto scratch = [&](size_t bytes) { return (rc = need_scratch(c, bytes)) == DSMC_OK ? c->scratch : nullptr; };
+    const cudaError_t e = dsmc::shadow_flux(npoint, spot, nface, facet, face_normal, za, tt, nmonte, F, scratch,
+                                            c->stream, &overflows, &c->last_kernel_ms);
+    if (rc != DSMC_OK) return rc;
+    DSMC_CUDA_TRY(c, e);
     if (overflows) return fail(c, DSMC_ERR_INVALID, "BVH deeper than the traversal stack");
     return DSMC_OK;
 }
@@ -663,17 +701,13 @@ int dsmc_velocity_record(dsmc_ctx *c, int64_t n, int per_bucket, int64_t total_c
     long long chunk = (256ll << 20) / (4 * nb);
     chunk = chunk < 256 ? 256 : chunk;
     if (chunk > n) chunk = n > 0 ? n : 1;
-    struct Bufs {
-        void *p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        ~Bufs() { for (void *q : p) if (q) cudaFree(q); }
-    } b;
     const long long slots = nb * per_bucket;
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[0], chunk * nb * sizeof(int)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[1], nb * sizeof(int)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[2], slots * 3 * sizeof(double)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[3], slots * sizeof(int)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[4], slots * sizeof(unsigned long long)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&b.p[5], chunk * sizeof(int)));
+    ScratchUse use(c);
+    for (size_t bytes : {chunk * nb * sizeof(int), nb * sizeof(int), slots * 3 * sizeof(double), slots * sizeof(int),
+                         slots * sizeof(unsigned long long), chunk * sizeof(int)})
+        use.part(bytes);
+    if ((rc = need_scratch(c, use.total)) != DSMC_OK) return rc;
+    struct { void *p[6]; } b = {{use.at(0), use.at(1), use.at(2), use.at(3), use.at(4), use.at(5)}};
     DSMC_CUDA_TRY(c, cudaMemsetAsync(b.p[1], 0, nb * sizeof(int), c->stream));
     dsmc::RecordArgs ra{};
     ra.rows = static_cast<int *>(b.p[0]);

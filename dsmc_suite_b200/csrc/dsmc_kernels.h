@@ -1,6 +1,8 @@
 // dsmc_kernels.h - host-side launchers of the DSMC kernels (internal to the library).
 #pragma once
 
+#include <functional>
+
 #include "dsmc_device.cuh"
 
 namespace dsmc {
@@ -47,9 +49,11 @@ cudaError_t launch_thermal(const ThermalSetup &s, const double *flux, const doub
 
 // Monte Carlo shadow flux (kernel_raytrace.cu): builds the BVH of the mesh on the host, traces
 // on `stream` and copies F [nface][tt] back (synchronous). *overflows counts traversal-stack
-// overflows (0 for meshes below 2^24 faces).
+// overflows (0 for meshes below 2^24 faces). scratch(bytes) gives device memory for the call, or
+// nullptr.
 cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *facet,
                         const double *normal, double za, int tt, int nmonte, double *F_host,
-                        cudaStream_t stream, long long *overflows, double *kernel_ms);
+                        const std::function<void *(size_t)> &scratch, cudaStream_t stream,
+                        long long *overflows, double *kernel_ms);
 
 }  // namespace dsmc

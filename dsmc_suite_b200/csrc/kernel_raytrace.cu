@@ -398,7 +398,8 @@ __global__ void __launch_bounds__(32 * kWarps) shadow_kernel(const ShadowArgs a)
 
 cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *facet,
                         const double *normal, double za, int tt, int nmonte, double *F_host,
-                        cudaStream_t stream, long long *overflows, double *kernel_ms) {
+                        const std::function<void *(size_t)> &scratch, cudaStream_t stream,
+                        long long *overflows, double *kernel_ms) {
     std::vector<float> V(3 * static_cast<size_t>(npoint));
     for (size_t k = 0; k < V.size(); k++) V[k] = static_cast<float>(spot[k]);
     Builder bld(V, facet, nface);
@@ -412,20 +413,21 @@ cudaError_t shadow_flux(int npoint, const double *spot, int nface, const int *fa
         tris[3 * k + 1] = make_float4(v1[0] - v0[0], v1[1] - v0[1], v1[2] - v0[2], 0.0f);
         tris[3 * k + 2] = make_float4(v2[0] - v0[0], v2[1] - v0[1], v2[2] - v0[2], 0.0f);
     }
-    struct Bufs {
-        void *p[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        ~Bufs() { for (void *q : p) if (q) cudaFree(q); }
-    } b;
     const size_t nn = bld.nodes.size(), nfc = static_cast<size_t>(nface), np = static_cast<size_t>(npoint);
     const size_t nF = nfc * static_cast<size_t>(tt);
+    // one block from the caller: nodes, triangles, faces, vertices, normals, F, overflow count
+    const size_t sizes[7] = {nn * sizeof(BvhNode), tris.size() * sizeof(float4), nfc * 3 * sizeof(int),
+                             np * 3 * sizeof(double), nfc * 3 * sizeof(double), nF * sizeof(double), sizeof(int)};
+    struct { void *p[7]; } b;
+    size_t at[7], total = 0;
+    for (int k = 0; k < 7; k++) {
+        at[k] = total;
+        total += (sizes[k] + 255) & ~size_t(255);
+    }
+    void *block = scratch(total);
+    if (!block) return cudaErrorMemoryAllocation;
+    for (int k = 0; k < 7; k++) b.p[k] = static_cast<char *>(block) + at[k];
     cudaError_t e;
-    if ((e = cudaMalloc(&b.p[0], nn * sizeof(BvhNode))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[1], tris.size() * sizeof(float4))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[2], nfc * 3 * sizeof(int))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[3], np * 3 * sizeof(double))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[4], nfc * 3 * sizeof(double))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[5], nF * sizeof(double))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&b.p[6], sizeof(int))) != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(b.p[0], bld.nodes.data(), nn * sizeof(BvhNode), cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b.p[1], tris.data(), tris.size() * sizeof(float4), cudaMemcpyHostToDevice, stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b.p[2], facet, nfc * 3 * sizeof(int), cudaMemcpyHostToDevice, stream)) != cudaSuccess ||

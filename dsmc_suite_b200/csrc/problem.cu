@@ -1,4 +1,5 @@
 // problem.cu - upload of one DSMC problem to the device (see problem.h).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -76,14 +77,37 @@ struct Uploader {
     size_t errlen;
 
     int alloc(void **p, size_t bytes) {
-        const cudaError_t e = !async ? cudaMalloc(p, bytes)
-                              : pr.pool ? cudaMallocFromPoolAsync(p, bytes, pr.pool, stream)
-                                        : cudaMallocAsync(p, bytes, stream);
+        size_t held = bytes;
+        if (!async) {
+            // the smallest spare block that fits without wasting more than it holds
+            size_t best = pr.spare.size();
+            for (size_t k = 0; k < pr.spare.size(); k++)
+                if (pr.spare[k].bytes >= bytes && pr.spare[k].bytes <= 2 * bytes + 4096 &&
+                    (best == pr.spare.size() || pr.spare[k].bytes < pr.spare[best].bytes))
+                    best = k;
+            if (best < pr.spare.size()) {
+                *p = pr.spare[best].p;
+                held = pr.spare[best].bytes;
+                pr.spare.erase(pr.spare.begin() + static_cast<long>(best));
+                pr.owned.push_back({*p, held});
+                pr.bytes += held;
+                return DSMC_OK;
+            }
+        }
+        cudaError_t e = !async ? cudaMalloc(p, bytes)
+                        : pr.pool ? cudaMallocFromPoolAsync(p, bytes, pr.pool, stream)
+                                  : cudaMallocAsync(p, bytes, stream);
+        if (e == cudaErrorMemoryAllocation && !async && !pr.spare.empty()) {
+            cudaGetLastError();   // room taken by blocks that did not fit
+            for (const Problem::Block &q : pr.spare) cudaFree(q.p);
+            pr.spare.clear();
+            e = cudaMalloc(p, bytes);
+        }
         if (e != cudaSuccess)
             return report(err, errlen, e == cudaErrorMemoryAllocation ? DSMC_ERR_NO_MEMORY : DSMC_ERR_CUDA,
                           "device allocation", e);
-        pr.owned.push_back(*p);
-        pr.bytes += bytes;
+        pr.owned.push_back({*p, held});
+        pr.bytes += held;
         return DSMC_OK;
     }
 
@@ -116,10 +140,20 @@ struct Uploader {
 }  // namespace
 
 void Problem::release() {
-    for (void *q : owned) {
-        if (async_alloc) cudaFreeAsync(q, stream);
-        else cudaFree(q);
+    for (const Block &q : owned) {
+        if (async_alloc) cudaFreeAsync(q.p, stream);
+        else cudaFree(q.p);
     }
+    for (const Block &q : spare) cudaFree(q.p);
+    owned.clear();
+    spare.clear();
+    bytes = 0;
+    t = DevTables{};
+}
+
+void Problem::recycle() {
+    if (async_alloc) return release();
+    spare.insert(spare.end(), owned.begin(), owned.end());
     owned.clear();
     bytes = 0;
     t = DevTables{};
@@ -176,7 +210,7 @@ int problem_build(Problem &pr, const dsmc_params *p, const dsmc_surface *s,
                   bool async_alloc, char *err, size_t errlen, cudaMemPool_t pool) {
     int rc = problem_check(p, s, col, err, errlen);
     if (rc != DSMC_OK) return rc;
-    pr.release();
+    pr.recycle();
     pr.async_alloc = async_alloc;
     pr.stream = stream;
     pr.pool = pool;
@@ -244,6 +278,15 @@ int problem_build(Problem &pr, const dsmc_params *p, const dsmc_surface *s,
     if ((rc = u.zeroed(static_cast<size_t>(pr.nhcell), &t.horizon)) != DSMC_OK) return rc;
     if (pr.nhist > 0 && (rc = u.zeroed(static_cast<size_t>(pr.nhist), &t.speed_hist)) != DSMC_OK) return rc;
     t.stats = stats;
+    // spare blocks beyond the bound, the largest first
+    std::sort(pr.spare.begin(), pr.spare.end(),
+              [](const Problem::Block &a, const Problem::Block &b) { return a.bytes < b.bytes; });
+    size_t kept = 0;
+    for (const Problem::Block &q : pr.spare) kept += q.bytes;
+    for (; kept > Problem::kSpareBytes; pr.spare.pop_back()) {
+        kept -= pr.spare.back().bytes;
+        cudaFree(pr.spare.back().p);
+    }
     // the host arrays of the caller are pageable: the copies above have been staged when the
     // calls returned, but wait for the device so that errors surface here
     const cudaError_t e = cudaStreamSynchronize(stream);

@@ -14,7 +14,9 @@ namespace dsmc {
 struct Problem {
     dsmc_params p{};
     DevTables t{};
-    std::vector<void *> owned;     // device allocations of this problem
+    struct Block { void *p; size_t bytes; };
+    std::vector<Block> owned;      // device allocations of this problem
+    std::vector<Block> spare;      // those of earlier problems, for problem_build to take
     long long ncell = 0, nhcell = 0, nhist = 0;
     size_t bytes = 0;              // device bytes held by the problem
     bool async_alloc = false;      // owned buffers are stream-ordered allocations on `stream`
@@ -25,7 +27,13 @@ struct Problem {
     Problem(const Problem &) = delete;
     Problem &operator=(const Problem &) = delete;
     ~Problem() { release(); }
+    // Frees everything. recycle() keeps plain allocations for the next problem_build, which takes
+    // those that fit and frees the rest down to kSpareBytes: an allocation and a release per table
+    // and set-up cost 0.1 ms, and now and then a stall of up to 100 ms while the driver returned
+    // and remapped memory.
     void release();
+    void recycle();
+    static constexpr size_t kSpareBytes = size_t(128) << 20;
 };
 
 // Device bytes a problem with these inputs would hold (grids, tables, histograms).
