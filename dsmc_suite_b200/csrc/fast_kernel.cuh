@@ -1295,6 +1295,23 @@ __device__ __forceinline__ void gravity(PosT<double> &q, double GM) {
     q.a[2] = g * q.z;
 }
 
+// The step's inside tests against the current cell's bounds. warp_kernel's unrolled steps keep only
+// their conjunction and repeat the three in the slow path: kept for it, each test cost a step an
+// instruction to hold (1e7 Ceres-like particles 281 against 278 ms).
+template <typename R>
+__device__ __forceinline__ bool in_shell(const PosT<R> &q, const BoundsT<R> &b) {
+    return (q.r2 > b.r2lo) & (q.r2 <= b.r2hi);
+}
+template <typename R>
+__device__ __forceinline__ bool in_row(const PosT<R> &q, const BoundsT<R> &b) {
+    const R zz = q.z * fabs(q.z);
+    return (zz > q.r2 * b.zlo) & (zz <= q.r2 * b.zhi);
+}
+template <typename R>
+__device__ __forceinline__ bool in_column(const PosT<R> &q, const BoundsT<R> &b) {
+    return (q.x * b.c0 - q.y * b.s0 > R(0)) & (q.x * b.c1 - q.y * b.s1 <= R(0));
+}
+
 template <typename R>
 __device__ __forceinline__ void start_pos(const HotT<R> &h, PosT<R> &q) {
     q.x = pos(h, 0);
@@ -1634,7 +1651,7 @@ enum Event { kEvNone = 0, kEvLanded, kEvEscaped, kEvCap, kEvEmpty, kEvResume };
 // the change's code runs once per iteration and not once per step (a warp of long hops changes a
 // cell on half of its steps), the branches per step halve, and the event code exists once.
 // A launch runs a.K / kUnroll iterations, so a lane takes at most a.K steps.
-// Measured at kUnroll 8: 1e7 Ceres-like particles 280.4 ms against 291.5 ms, 3e5 of the reference
+// Measured at kUnroll 8: 1e7 Ceres-like particles 278 ms against 291.5 ms, 3e5 of the reference
 // model 72 against 103 ms; 4 and 12 steps in a row ran the former in 307 and 297 ms. Few particles,
 // whose warps have nothing to hide a branch behind: 512 Ceres-like 1.60 ms at 12 steps in a row,
 // 1.77 at 8, 3.4 in fast_kernel; 500 of the reference model with collisions 42.9 ms at 12, 46.7 at
@@ -1730,7 +1747,6 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
             if (last || !__any_sync(kAll, flying)) break;
         }
         R d[3];
-        bool in_r = true, in_t = true, in_f = true;
         bool left = false, struck = false;
         auto settle = [&]() {   // a step's photolysis and deposit, once the cell is known
             const bool day = M::kRef ? ((h.cell & 0xff) < k.half_ffd)
@@ -1754,11 +1770,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
                 verlet_step(h, q, k.dt, k.c1, k.c2, d);
                 gravity(q, k.GM);
                 taken++;
-                const R zz = q.z * fabs(q.z);
-                in_r = (q.r2 > b.r2lo) & (q.r2 <= b.r2hi);
-                in_t = (zz > q.r2 * b.zlo) & (zz <= q.r2 * b.zhi);
-                in_f = (q.x * b.c0 - q.y * b.s0 > R(0)) & (q.x * b.c1 - q.y * b.s1 <= R(0));
-                if (!(in_r & in_t & in_f)) {
+                if (!(in_shell(q, b) & in_row(q, b) & in_column(q, b))) {
                     left = true;
                     break;
                 }
@@ -1773,7 +1785,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
                 event = kEvLanded;
             } else if (q.r2 >= k.re2) {
                 event = kEvEscaped;
-            } else if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+            } else if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_shell(q, b),
+                                            in_row(q, b), in_column(q, b)) &&
                        kMode == 1 && q.r2 != q.r2) {
                 taken = drift_nowhere(h, taken, n);
             } else {
