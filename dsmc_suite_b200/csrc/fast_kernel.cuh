@@ -14,6 +14,9 @@
 // (cell change, launch, landing, collision, end of life) leave the loop for code that reads the
 // boundary tables and the cold per-particle fields.
 //
+// Two loops share the pieces: fast_kernel, whose lanes run free of one another, and warp_kernel,
+// whose lanes step together.
+//
 // Included by the translation units that instantiate it (fast_served.cu, fast_one32.cu,
 // fast_one64.cu), one per family of kernels so that they compile side by side.
 #pragma once
@@ -1321,9 +1324,10 @@ __device__ __forceinline__ void start_pos(const HotT<R> &h, PosT<R> &q) {
 }
 
 // One Verlet step of the reference's variant. FP32: (hi, lo) position and velocity sums, and the
-// acceleration carried as the velocity change -a * dt (c1 = 1.5 dt, c2 = dt / 6; three multiplies fewer per step, and at a power-of-two dt the same roundings as
-// a and dt kept apart); FP64: plain doubles with c1 = 1.5 dt^2, c2 = dt^2 / 6. q holds the current
-// position on entry and the new one on exit; d the displacement.
+// acceleration carried as the velocity change -a * dt (c1 = 1.5 dt, c2 = dt / 6; three multiplies
+// fewer per step, and at a power-of-two dt the same roundings as a and dt kept apart); FP64: plain
+// doubles with c1 = 1.5 dt^2, c2 = dt^2 / 6. q holds the current position on entry and the new one
+// on exit; d the displacement.
 // The FP32 update runs in packed pairs: x and y of a vector side by side, and for z the position
 // and velocity sums side by side. The acceleration keeps its minus sign because packed operands
 // take no negation. 1e7 Ceres-like particles: 2.23e11 -> 2.32e11 particle-steps/s, 3e6

@@ -1,6 +1,6 @@
 // kernel_thermal.cu - the thermal model that feeds the DSMC phases (src/thermal/thermal_model.c
-// of the reference), one GPU thread per surface column. Compiled with -fmad=false: the column
-// arithmetic follows the reference's FP64 operation order, so the Crank-Nicolson steps and the
+// of the reference), eight lanes or one thread per surface column. Compiled with -fmad=false: the
+// column arithmetic follows the reference's FP64 operation order, so the Crank-Nicolson steps and the
 // Thomas sweeps are bit-identical to the CPU's; only CUDA's log10 / pow / sqrt inside the surface
 // energy balance may round differently in the last place from glibc's.
 //
