@@ -128,7 +128,10 @@ __device__ double surface_temperature(const ThermalArgs &a, double F, double oT)
     return (T0 + T1) / 2.0;
 }
 
-// One implicit step of a column with its profile in q and scratch d, element i at [i * n].
+// One implicit step of a column with its profile in q and scratch d, element i at [i * n]. kGroup lanes
+// (all of the warp's groups together) work on one q and d: the step overwrites the old profile once
+// every lane has read it, and the next step reads the new one once every lane has written it.
+template <int kGroup>
 __device__ __forceinline__ void diffuse(const ThermalArgs &a, const double *cp, const double *piv,
                                         const double *rcp, double *q, double *d, long long n, double Ts) {
     constexpr int kAhead = 8;   // depths read before the chain needs them
@@ -159,6 +162,7 @@ __device__ __forceinline__ void diffuse(const ThermalArgs &a, const double *cp, 
             }
     }
     dprev = divide(0.0 - a.a_last * dprev, piv[h - 1], rcp[h - 1]);
+    if (kGroup > 1) __syncwarp();
     // back substitution, overwriting the profile
     double x = dprev;
     q[(h - 1) * n] = x;
@@ -177,6 +181,7 @@ __device__ __forceinline__ void diffuse(const ThermalArgs &a, const double *cp, 
                 q[(i - j) * n] = x;
             }
     }
+    if (kGroup > 1) __syncwarp();
 }
 
 // Columns in device memory, one thread each.
@@ -191,7 +196,7 @@ __global__ void thermal_column_kernel(const ThermalArgs a) {
         for (int d = 0; d < a.h; d++) qT[d * n] = a.T_init[c];
     for (int step = 0; step < a.n_sub; step++) {
         const double Ts = surface_temperature<1>(a, F, mine ? qT[n] : a.T_init[c]);
-        if (mine) diffuse(a, a.cp, a.piv, a.rcp, qT, dp, n, Ts);
+        if (mine) diffuse<1>(a, a.cp, a.piv, a.rcp, qT, dp, n, Ts);
     }
     if (mine) a.T_surface[c] = qT[0];
 }
@@ -199,8 +204,8 @@ __global__ void thermal_column_kernel(const ThermalArgs a) {
 extern __shared__ double thermal_smem[];
 
 // Columns in shared memory, kGroup lanes each: [cp | piv | rcp] of h, then the profiles and d' of
-// the block's columns, [h][columns]. Every lane of a group stores the same values, so it reads
-// back only what it wrote itself.
+// the block's columns, [h][columns]. Every lane of a group reads and writes the whole column, all the
+// same values; the warp meets wherever one lane would write what another has still to read.
 template <int kGroup>
 __global__ void thermal_shared_kernel(const ThermalArgs a) {
     const int h = a.h, cols = blockDim.x / kGroup, own = threadIdx.x / kGroup;
@@ -216,8 +221,9 @@ __global__ void thermal_shared_kernel(const ThermalArgs a) {
     const int c = min(col, a.ncol - 1);   // the groups past the end repeat the last column
     const double F = a.flux[c], T_init = a.T_init[c];
     for (int i = 0; i < h; i++) q[i * cols] = T_init;
+    __syncwarp();
     for (int step = 0; step < a.n_sub; step++)
-        diffuse(a, cp, piv, rcp, q, d, cols, surface_temperature<kGroup>(a, F, q[cols]));
+        diffuse<kGroup>(a, cp, piv, rcp, q, d, cols, surface_temperature<kGroup>(a, F, q[cols]));
     if (col < a.ncol && threadIdx.x % kGroup == 0) a.T_surface[c] = q[0];
 }
 
