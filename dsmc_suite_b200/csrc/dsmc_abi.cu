@@ -38,6 +38,10 @@ struct dsmc_ctx {
     double last_kernel_ms = 0.0;     // device time of the last thermal / shadow-flux kernel
     void *scratch = nullptr;          // device scratch of the synchronous calls (need_scratch)
     size_t scratch_bytes = 0;
+    // the end of the work issued on each stream that the context was given, but its own (note_work)
+    std::vector<cudaEvent_t> used;
+    int used_now = -1;               // that of the current stream, -1: none yet
+    bool unseen = false;             // work whose end no event tells: part of a graph of the caller's
     char err[512] = {0};
 };
 
@@ -83,6 +87,45 @@ void free_outputs(dsmc_ctx *c) {
     c->t.steps = nullptr;
     c->t.out_cap = 0;
     c->t.out_base = 0;
+}
+
+// After work is issued on the current stream. Buffers that a later call takes over may be in use by
+// asynchronous work on streams the context was given earlier, and such a stream may be gone by then,
+// so an event of the context's own, recorded behind the work, stands for it. The context's own stream
+// outlives its work and needs one only when the context leaves it (dsmc_ctx_set_stream).
+void note_work(dsmc_ctx *c) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(c->stream, &cap);
+    if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) {
+        c->unseen = true;
+        return;
+    }
+    for (size_t k = 0; e == cudaSuccess && c->used_now < 0 && k < c->used.size(); k++)
+        if (cudaEventQuery(c->used[k]) == cudaSuccess) c->used_now = static_cast<int>(k);
+    if (e == cudaSuccess && c->used_now < 0) {
+        cudaEvent_t ev = nullptr;
+        e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (e == cudaSuccess) {
+            c->used_now = static_cast<int>(c->used.size());
+            c->used.push_back(ev);
+        }
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(c->used[c->used_now], c->stream);
+    cudaGetLastError();   // of the query, or an error that leaves the work unseen
+    if (e != cudaSuccess) c->unseen = true;
+}
+
+void note_foreign_work(dsmc_ctx *c) {
+    if (c->stream != c->own_stream) note_work(c);
+}
+
+// Waits for the work of this context, on every stream, and for no other work.
+cudaError_t finish_work(dsmc_ctx *c) {
+    for (cudaEvent_t ev : c->used) {
+        const cudaError_t e = cudaEventSynchronize(ev);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaStreamSynchronize(c->stream);
 }
 
 // Device scratch of at least `bytes` bytes, kept by the context up to kScratchKept bytes (a call
@@ -182,6 +225,7 @@ int dsmc_ctx_destroy(dsmc_ctx *c) {
     free_outputs(c);
     if (c->stats) cudaFree(c->stats);
     if (c->scratch) cudaFree(c->scratch);
+    for (cudaEvent_t ev : c->used) cudaEventDestroy(ev);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return DSMC_OK;
@@ -189,7 +233,14 @@ int dsmc_ctx_destroy(dsmc_ctx *c) {
 
 int dsmc_ctx_set_stream(dsmc_ctx *c, void *stream) {
     if (!c) return DSMC_ERR_INVALID;
-    c->stream = stream ? static_cast<cudaStream_t>(stream) : c->own_stream;
+    const cudaStream_t to = stream ? static_cast<cudaStream_t>(stream) : c->own_stream;
+    if (c->stream == c->own_stream && to != c->stream) {
+        const int rc = set_device(c);
+        if (rc != DSMC_OK) return rc;
+        note_work(c);
+    }
+    c->stream = to;
+    c->used_now = -1;   // even for the same handle: it may name another stream by now
     return DSMC_OK;
 }
 
@@ -230,12 +281,13 @@ int dsmc_enable_particle_outputs(dsmc_ctx *c, int64_t n) {
     if (!c || n < 0) return DSMC_ERR_INVALID;
     int rc = set_device(c);
     if (rc != DSMC_OK) return rc;
-    DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    if (n > 0 && n == c->t.out_cap) {   // the same rows again: cleared, as new ones are
+    DSMC_CUDA_TRY(c, finish_work(c));
+    if (n > 0 && n == c->t.out_cap && !c->unseen) {   // the same rows again: cleared, as new ones are
         c->t.out_base = 0;
         DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[0], 0, static_cast<size_t>(n) * 9 * sizeof(double), c->stream));
         DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[1], 0, static_cast<size_t>(n) * sizeof(int), c->stream));
         DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[2], 0, static_cast<size_t>(n) * sizeof(long long), c->stream));
+        note_foreign_work(c);
         return DSMC_OK;
     }
     free_outputs(c);
@@ -250,6 +302,7 @@ int dsmc_enable_particle_outputs(dsmc_ctx *c, int64_t n) {
     c->t.fate = static_cast<int *>(c->outputs[1]);
     c->t.steps = static_cast<long long *>(c->outputs[2]);
     c->t.out_cap = n;
+    note_foreign_work(c);
     return DSMC_OK;
 }
 
@@ -268,6 +321,7 @@ int dsmc_zero(dsmc_ctx *c) {
         DSMC_CUDA_TRY(c, cudaMemsetAsync(c->t.fate, 0, c->t.out_cap * sizeof(int), c->stream));
         DSMC_CUDA_TRY(c, cudaMemsetAsync(c->t.steps, 0, c->t.out_cap * sizeof(long long), c->stream));
     }
+    note_foreign_work(c);
     return DSMC_OK;
 }
 
@@ -282,6 +336,7 @@ int dsmc_run(dsmc_ctx *c, int path, int64_t pid_begin, int64_t n) {
     switch (path) {
         case DSMC_PATH_PLAIN_FP64:
             DSMC_CUDA_TRY(c, dsmc::launch_plain_fp64(c->params, c->t, pid_begin, n, c->num_sms, c->stream));
+            note_foreign_work(c);
             c->last_launches = n > 0 ? 1 : 0;
             return DSMC_OK;
         case DSMC_PATH_FAST_FP64:
@@ -296,9 +351,11 @@ int dsmc_run(dsmc_ctx *c, int path, int64_t pid_begin, int64_t n) {
             cudaError_t e = c->fast->run(c->params, c->t, path == DSMC_PATH_FAST_FP64, pid_begin, n,
                                          c->num_sms, c->stream);
             c->last_launches = c->fast->launches;
-            if (e != cudaSuccess)
+            if (e != cudaSuccess) {
+                note_foreign_work(c);   // launches may still run
                 return fail(c, e == cudaErrorMemoryAllocation ? DSMC_ERR_NO_MEMORY : DSMC_ERR_CUDA,
                             "fast path: %s", cudaGetErrorString(e));
+            }
             return DSMC_OK;
         }
         default:
@@ -436,6 +493,7 @@ int dsmc_copy_grids_device(dsmc_ctx *c, uint64_t *density_dst, uint64_t *horizon
         DSMC_CUDA_TRY(c, cudaMemcpyAsync(density_dst, c->t.density, c->ncell * sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->stream));
     if (horizon_dst)
         DSMC_CUDA_TRY(c, cudaMemcpyAsync(horizon_dst, c->t.horizon, c->nhcell * sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->stream));
+    note_foreign_work(c);
     return DSMC_OK;
 }
 

@@ -1,0 +1,68 @@
+"""The library's host code on a fake CUDA runtime (fake_cudart.cpp): which streams, allocations and
+attributes a call uses, and what it does when an allocation fails. No kernel runs, so nothing here
+looks at results; the GPU tests do."""
+from __future__ import annotations
+
+import ctypes as C
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def fake_lib(built, tmp_path_factory):
+    """The built objects linked with the fake runtime, as a library of their own."""
+    from dsmc_suite_b200 import _native as N
+    from dsmc_suite_b200 import build as B
+    so = tmp_path_factory.mktemp("fake") / "libdsmc_fake.so"
+    objs = [str(B.OBJ / (s + ".o")) for s in [*B.CUDA_SOURCES, *B.C_SOURCES]]
+    # -Bsymbolic: the library's calls go to the fake even where a real runtime is loaded
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
+                    "-o", str(so), str(ROOT / "tests" / "fake_cudart.cpp"), *objs, "-lm", "-lpthread"],
+                   check=True, capture_output=True)
+    L = C.CDLL(str(so))
+    for name, res, args in N.SIGNATURES:
+        f = getattr(L, name)
+        f.restype, f.argtypes = res, args
+    for name in ("allocs", "loops", "reads", "races", "device_syncs", "lowered"):
+        getattr(L, "fake_" + name).restype = C.c_longlong
+    L.fake_held.restype = C.c_size_t
+    L.fake_stream.restype = C.c_void_p
+    L.fake_limit.argtypes = [C.c_size_t]
+    L.fake_fail_at.argtypes = L.fake_finish_after.argtypes = [C.c_longlong]
+    return L
+
+
+@pytest.fixture
+def fake(fake_lib, N, monkeypatch):
+    monkeypatch.setattr(N, "_lib", fake_lib)
+    fake_lib.fake_reset()
+    return fake_lib
+
+
+@pytest.fixture
+def context(fake):
+    from dsmc_suite_b200 import Context
+    with Context(0) as c:
+        yield c
+
+
+@pytest.fixture(scope="module")
+def problem(N):
+    ico = N.Icosphere(2)
+    return N.params_config(N.RUNNER_BALLISTIC, hd=20), N.SurfaceInputs(ico=ico, face_T=ico.face_temperature())
+
+
+def test_rows_are_cleared_after_the_run_that_writes_them(fake, context, N, problem):
+    """A plain run is asynchronous; the same rows enabled again on another stream are cleared only
+    after it, whether that stream is the context's own or one more of the caller's."""
+    context.setup(*problem)
+    context.enable_particle_outputs(100)
+    for stream in (fake.fake_stream(), None, fake.fake_stream(), fake.fake_stream()):
+        context.run(N.PATH_PLAIN_FP64, 0, 100)
+        context.set_stream(stream)
+        context.enable_particle_outputs(100)
+        assert fake.fake_races() == 0
