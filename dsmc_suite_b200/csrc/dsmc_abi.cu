@@ -42,6 +42,7 @@ struct dsmc_ctx {
     std::vector<cudaEvent_t> used;
     int used_now = -1;               // that of the current stream, -1: none yet
     bool unseen = false;             // work whose end no event tells: part of a graph of the caller's
+    bool lent = false;               // the caller has the address of a grid of this problem
     char err[512] = {0};
 };
 
@@ -250,10 +251,12 @@ int dsmc_setup(dsmc_ctx *c, const dsmc_params *p, const dsmc_surface *s,
     int rc = dsmc::problem_check(p, s, col, c->err, sizeof c->err);
     if (rc != DSMC_OK) return rc;
     if ((rc = set_device(c)) != DSMC_OK) return rc;
-    // nothing may still read the tables that the new problem takes over, on any stream the context
-    // was given
-    DSMC_CUDA_TRY(c, cudaDeviceSynchronize());
+    // nothing may still use the blocks that the new problem takes over. Blocks that work unknown to
+    // the context may use are freed instead, which waits for the device.
+    DSMC_CUDA_TRY(c, finish_work(c));
     c->ready = false;
+    if (c->lent || c->unseen) c->prob.release();
+    c->lent = false;
     rc = dsmc::problem_build(c->prob, p, s, col, c->stats, c->stream, false, c->err, sizeof c->err);
     if (rc != DSMC_OK) {
         free_tables(c);
@@ -500,6 +503,7 @@ int dsmc_copy_grids_device(dsmc_ctx *c, uint64_t *density_dst, uint64_t *horizon
 int dsmc_density_device(dsmc_ctx *c, uint64_t **dev_ptr, int64_t *ncell) {
     if (!c || !dev_ptr || !ncell) return DSMC_ERR_INVALID;
     if (!c->ready) return fail(c, DSMC_ERR_STATE, "no problem set up");
+    c->lent = true;
     *dev_ptr = reinterpret_cast<uint64_t *>(c->t.density);
     *ncell = c->ncell;
     return DSMC_OK;
@@ -508,6 +512,7 @@ int dsmc_density_device(dsmc_ctx *c, uint64_t **dev_ptr, int64_t *ncell) {
 int dsmc_horizon_device(dsmc_ctx *c, uint64_t **dev_ptr, int64_t *ncell) {
     if (!c || !dev_ptr || !ncell) return DSMC_ERR_INVALID;
     if (!c->ready) return fail(c, DSMC_ERR_STATE, "no problem set up");
+    c->lent = true;
     *dev_ptr = reinterpret_cast<uint64_t *>(c->t.horizon);
     *ncell = c->nhcell;
     return DSMC_OK;

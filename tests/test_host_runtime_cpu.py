@@ -66,3 +66,39 @@ def test_rows_are_cleared_after_the_run_that_writes_them(fake, context, N, probl
         context.set_stream(stream)
         context.enable_particle_outputs(100)
         assert fake.fake_races() == 0
+
+
+def test_setup_waits_for_its_own_work_alone(fake, context, N, problem):
+    """A set-up reuses the blocks of the problem before it once that problem's work has ended, on
+    every stream the context was given; it does not wait for the device, which CUDA refuses while
+    another thread captures a stream (as a server does when it opens)."""
+    from dsmc_suite_b200 import Context
+    fake.fake_capturing(1)
+    context.setup(*problem)
+    for stream in (fake.fake_stream(), fake.fake_stream(), None):
+        context.run(N.PATH_PLAIN_FP64, 0, 100)
+        context.set_stream(stream)
+        before = fake.fake_allocs()
+        context.setup(*problem)
+        assert fake.fake_allocs() == before and fake.fake_races() == 0
+    with Context(0) as other:
+        other.setup(*problem)
+        other.run(N.PATH_PLAIN_FP64, 0, 100)
+        context.setup(*problem)
+        assert fake.fake_races() > 0   # the other context's kernel still runs, and is not waited for
+    assert fake.fake_device_syncs() == 0
+
+
+def test_setup_leaves_grids_it_handed_out(fake, context, N, problem):
+    """The caller may be reading a grid whose device address it was given, on a stream the context
+    does not know: those blocks are freed, which waits for the device, and not written again."""
+    context.setup(*problem)
+    before = fake.fake_allocs()
+    context.setup(*problem)
+    assert fake.fake_allocs() == before
+    context.density_device()
+    context.setup(*problem)
+    assert fake.fake_allocs() > before
+    before = fake.fake_allocs()
+    context.setup(*problem)
+    assert fake.fake_allocs() == before
