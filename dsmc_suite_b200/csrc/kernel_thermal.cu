@@ -229,7 +229,7 @@ __global__ void thermal_shared_kernel(const ThermalArgs a) {
 
 constexpr int kGroup = 8;
 
-constexpr size_t kSharedPerSm = 227 * 1024;
+constexpr size_t kSharedPerSm = 227 * 1024;   // of an SM, and of a block at most
 
 size_t shared_bytes(int h, int cols) { return static_cast<size_t>(h) * (3 + 2 * cols) * sizeof(double); }
 
@@ -275,10 +275,11 @@ cudaError_t launch_thermal(const ThermalSetup &s, const double *flux, const doub
     a.T_surface = T_surface;
     const int cols = shared_cols(s.h, s.ncol, num_sms);
     if (cols) {
-        const size_t smem = shared_bytes(s.h, cols);
-        const cudaError_t e = cudaFuncSetAttribute(thermal_shared_kernel<kGroup>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        // the limit belongs to the function, which other threads launch too: always the largest
+        const cudaError_t e = cudaFuncSetAttribute(thermal_shared_kernel<kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(kSharedPerSm));
         if (e != cudaSuccess) return e;
+        const size_t smem = shared_bytes(s.h, cols);
         thermal_shared_kernel<kGroup><<<(s.ncol + cols - 1) / cols, cols * kGroup, smem, stream>>>(a);
         return cudaGetLastError();
     }

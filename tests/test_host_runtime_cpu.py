@@ -102,3 +102,15 @@ def test_setup_leaves_grids_it_handed_out(fake, context, N, problem):
     before = fake.fake_allocs()
     context.setup(*problem)
     assert fake.fake_allocs() == before
+
+
+def test_thermal_calls_leave_the_shared_memory_limit_alone(fake, context, N):
+    """The limit belongs to the function on the device, not to the call: a call of a shallow column
+    on one thread must not lower it between another thread's setting and its launch."""
+    from dsmc_suite_b200 import Context
+    tp = N.ThermalParams.default()
+    with Context(0) as other:
+        for ctx, depth in ((context, 0.05), (other, 0.02), (context, 0.12), (other, 0.05)):
+            tp.depth = depth
+            ctx.thermal(6, 12, tp)
+    assert fake.fake_lowered() == 0
