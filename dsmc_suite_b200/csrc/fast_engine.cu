@@ -34,7 +34,6 @@ void FastEngine::free_all() {
     d_ctr_ = nullptr;
     if (h_ctr_) cudaFreeHost(h_ctr_);
     h_ctr_ = nullptr;
-    if (d_map_) cudaFree(d_map_);
     d_map_ = nullptr;
     for (cudaEvent_t &e : round_) {
         if (e) cudaEventDestroy(e);
@@ -146,7 +145,6 @@ cudaError_t build_face_tables(const DevTables &t, float4 *out, cudaStream_t stre
 
 cudaError_t FastEngine::ensure_slots(int num_sms) {
     num_sms_ = num_sms;
-    num_sms_ = num_sms;
     // one wave: as many blocks per SM as can be resident together
     int resident = 0;
     cudaError_t e0;
@@ -163,27 +161,33 @@ cudaError_t FastEngine::ensure_slots(int num_sms) {
     if (resident < 1) return cudaErrorInvalidConfiguration;
     const int per_sm = (blocks_per_sm > resident || blocks_per_sm < 1) ? resident : blocks_per_sm;
     const long long want = static_cast<long long>(num_sms) * per_sm * block;
+    // each part by itself, so that a call after one whose allocation failed goes on where that stopped
+    cudaError_t e;
+    if (!d_ctr_ && (e = cudaMalloc(&d_ctr_, sizeof(FastCounters))) != cudaSuccess) return e;
+    if (!h_ctr_ && (e = cudaMallocHost(&h_ctr_, 3 * sizeof(FastCounters))) != cudaSuccess) return e;
+    for (cudaEvent_t &r : round_)
+        if (!r && (e = cudaEventCreateWithFlags(&r, cudaEventDisableTiming)) != cudaSuccess) return e;
     if (slot_mem_ && nslots_ == want && slot_fp64_ == fp64_) return cudaSuccess;
     free_graphs();
-    if (slot_mem_) { cudaFree(slot_mem_); slot_mem_ = nullptr; }
-    if (d_map_) { cudaFree(d_map_); d_map_ = nullptr; }
+    if (slot_mem_) cudaFree(slot_mem_);
+    slot_mem_ = nullptr;
+    nslots_ = 0;
     const long long S = want;
-    cudaError_t e = cudaMalloc(&slot_mem_, fast_slot_bytes(S, fp64_));
-    if (e != cudaSuccess) return e;
+    // behind the slots, the map of the drain's last launches (see drain): a counter, then one slot
+    // per thread
+    const size_t slot_bytes = (fast_slot_bytes(S, fp64_) + 255) & ~static_cast<size_t>(255);
+    if ((e = cudaMalloc(&slot_mem_, slot_bytes + (S + 32) * sizeof(int))) != cudaSuccess) {
+        slot_mem_ = nullptr;
+        return e;
+    }
+    d_map_ = reinterpret_cast<int *>(static_cast<char *>(slot_mem_) + slot_bytes);
     slots_ = Slots{};
     slots64_ = SlotsT<double>{};
     if (fp64_) slots64_ = carve_slots<double>(slot_mem_, S);
     else slots_ = carve_slots<float>(slot_mem_, S);
     slot_fp64_ = fp64_;
     nslots_ = S;
-    if (!d_ctr_) {
-        if ((e = cudaMalloc(&d_ctr_, sizeof(FastCounters))) != cudaSuccess) return e;
-        if ((e = cudaMallocHost(&h_ctr_, 3 * sizeof(FastCounters))) != cudaSuccess) return e;
-        for (cudaEvent_t &r : round_)
-            if ((e = cudaEventCreateWithFlags(&r, cudaEventDisableTiming)) != cudaSuccess) return e;
-    }
-    // the map of the drain's last launches (see drain): a counter, then one slot per thread
-    return cudaMalloc(&d_map_, (S + 32) * sizeof(int));
+    return cudaSuccess;
 }
 
 namespace {
@@ -516,6 +520,7 @@ cudaError_t FastEngine::serve_open(int num_sms, int max_instances, cudaStream_t 
     if (max_instances > ninst_cap_) {
         if (d_inst_) cudaFree(d_inst_);
         d_inst_ = nullptr;
+        ninst_cap_ = 0;
         if ((e = cudaMalloc(&d_inst_, static_cast<size_t>(max_instances) * sizeof(FastInst))) != cudaSuccess) return e;
         ninst_cap_ = max_instances;
         free_graphs();

@@ -315,7 +315,7 @@ private:
     FastCounters *d_ctr_ = nullptr;
     FastCounters *h_ctr_ = nullptr;           // [3] pinned: the last two launches', the start's
     cudaEvent_t round_[2] = {nullptr, nullptr};
-    int *d_map_ = nullptr;                    // packed slots of a drain's last launches
+    int *d_map_ = nullptr;                    // packed slots of a drain's last launches, in slot_mem_
     cudaGraphExec_t graph_mode_[3] = {nullptr, nullptr, nullptr};   // serving: loops 0, 1, 2
     int num_sms_ = 0;
     int variant_ = 4;

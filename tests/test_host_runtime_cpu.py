@@ -114,3 +114,26 @@ def test_thermal_calls_leave_the_shared_memory_limit_alone(fake, context, N):
             tp.depth = depth
             ctx.thermal(6, 12, tp)
     assert fake.fake_lowered() == 0
+
+
+@pytest.mark.parametrize("n", [200, 200_000])   # fewer particles than slots, and more
+def test_a_solve_after_one_whose_allocation_failed(fake, N, problem, n):
+    """Every device allocation of a first solve fails in turn: that call reports it, and the next call
+    on the same context solves as a first one does."""
+    from dsmc_suite_b200 import Context
+    for path in (N.PATH_FAST_FP32, N.PATH_FAST_FP64):
+        failed = 0
+        for k in range(64):
+            with Context(0) as ctx:
+                ctx.setup(*problem)
+                fake.fake_fail_at(k)
+                fake.fake_finish_after(2)
+                status = N.lib().dsmc_run(ctx.h, path, 0, n)
+                fake.fake_fail_at(-1)
+                if status == 0:
+                    break
+                assert status == -4
+                failed += 1
+                fake.fake_finish_after(2)
+                ctx.run(path, 0, n)
+        assert failed >= 3   # slots, counters, tables
