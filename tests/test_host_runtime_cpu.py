@@ -137,3 +137,18 @@ def test_a_solve_after_one_whose_allocation_failed(fake, N, problem, n):
                 fake.fake_finish_after(2)
                 ctx.run(path, 0, n)
         assert failed >= 3   # slots, counters, tables
+
+
+def test_large_thermal_solves_keep_their_device_block(fake, context, N):
+    """A thermal solve above the 256 MB that every call's scratch is kept up to allocates once per
+    context, also with other calls between."""
+    tp = N.ThermalParams.default()
+    tp.n_substep, tp.depth = 8, 0.1
+    h = context.thermal(120, 180, tp)[1]
+    assert 120 * 180 * h * 16 > 256 << 20
+    before, held = fake.fake_allocs(), fake.fake_held()
+    for k in range(3):
+        context.thermal(120, 180, tp)
+        context.fit_hist(np.ones((50, 8), dtype=np.uint64), 25.0, 3)
+        context.thermal(7, 9)
+    assert fake.fake_allocs() == before and fake.fake_held() == held
