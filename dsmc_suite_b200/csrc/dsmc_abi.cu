@@ -129,6 +129,27 @@ cudaError_t finish_work(dsmc_ctx *c) {
     return cudaStreamSynchronize(c->stream);
 }
 
+// Gives back what the context keeps for later calls: spare blocks of earlier problems, the scratch.
+// Returns whether there was any.
+bool give_back(dsmc_ctx *c) {
+    const bool any = c->scratch || !c->prob.spare.empty();
+    c->prob.release_spare();
+    if (c->scratch) cudaFree(c->scratch);
+    c->scratch = nullptr;
+    c->scratch_bytes = 0;
+    return any;
+}
+
+// cudaMalloc that makes room out of what the context keeps.
+cudaError_t device_alloc(dsmc_ctx *c, void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back(c)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 // Device scratch of at least `bytes` bytes, kept by the context up to scratch_keep bytes (a call that
 // needed more gives it back: ScratchUse): 256 MB, or what its largest thermal solve took, since a
 // program that solves such a grid solves it again and again (180 x 360 columns of 1044 depths, 1.1 GB:
@@ -140,7 +161,7 @@ int need_scratch(dsmc_ctx *c, size_t bytes) {
     if (c->scratch) cudaFree(c->scratch);
     c->scratch = nullptr;
     c->scratch_bytes = 0;
-    DSMC_CUDA_TRY(c, cudaMalloc(&c->scratch, bytes));
+    DSMC_CUDA_TRY(c, device_alloc(c, &c->scratch, bytes));
     c->scratch_bytes = bytes;
     return DSMC_OK;
 }
@@ -258,7 +279,9 @@ int dsmc_setup(dsmc_ctx *c, const dsmc_params *p, const dsmc_surface *s,
     c->ready = false;
     if (c->lent || c->unseen) c->prob.release();
     c->lent = false;
-    rc = dsmc::problem_build(c->prob, p, s, col, c->stats, c->stream, false, c->err, sizeof c->err);
+    auto build = [&] { return dsmc::problem_build(c->prob, p, s, col, c->stats, c->stream, false, c->err, sizeof c->err); };
+    rc = build();
+    if (rc == DSMC_ERR_NO_MEMORY && give_back(c)) rc = build();
     if (rc != DSMC_OK) {
         free_tables(c);
         return rc;
@@ -296,9 +319,9 @@ int dsmc_enable_particle_outputs(dsmc_ctx *c, int64_t n) {
     }
     free_outputs(c);
     if (n == 0) return DSMC_OK;
-    DSMC_CUDA_TRY(c, cudaMalloc(&c->outputs[0], static_cast<size_t>(n) * 9 * sizeof(double)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&c->outputs[1], static_cast<size_t>(n) * sizeof(int)));
-    DSMC_CUDA_TRY(c, cudaMalloc(&c->outputs[2], static_cast<size_t>(n) * sizeof(long long)));
+    DSMC_CUDA_TRY(c, device_alloc(c, &c->outputs[0], static_cast<size_t>(n) * 9 * sizeof(double)));
+    DSMC_CUDA_TRY(c, device_alloc(c, &c->outputs[1], static_cast<size_t>(n) * sizeof(int)));
+    DSMC_CUDA_TRY(c, device_alloc(c, &c->outputs[2], static_cast<size_t>(n) * sizeof(long long)));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[0], 0, static_cast<size_t>(n) * 9 * sizeof(double), c->stream));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[1], 0, static_cast<size_t>(n) * sizeof(int), c->stream));
     DSMC_CUDA_TRY(c, cudaMemsetAsync(c->outputs[2], 0, static_cast<size_t>(n) * sizeof(long long), c->stream));
@@ -352,8 +375,14 @@ int dsmc_run(dsmc_ctx *c, int path, int64_t pid_begin, int64_t n) {
             if (path == DSMC_PATH_FAST_FP64 && c->fast->block != 128)
                 return fail(c, DSMC_ERR_INVALID, "FAST_FP64 runs 128-thread blocks (launch shape has %d)",
                             c->fast->block);
-            cudaError_t e = c->fast->run(c->params, c->t, path == DSMC_PATH_FAST_FP64, pid_begin, n,
-                                         c->num_sms, c->stream);
+            auto solve = [&] {
+                return c->fast->run(c->params, c->t, path == DSMC_PATH_FAST_FP64, pid_begin, n, c->num_sms, c->stream);
+            };
+            cudaError_t e = solve();
+            if (e == cudaErrorMemoryAllocation && c->fast->launches == 0 && give_back(c)) {
+                cudaGetLastError();
+                e = solve();
+            }
             c->last_launches = c->fast->launches;
             if (e != cudaSuccess) {
                 note_foreign_work(c);   // launches may still run

@@ -491,6 +491,7 @@ cudaError_t FastEngine::drain(long long total, cudaStream_t stream) {
 
 cudaError_t FastEngine::run(const dsmc_params &p, const DevTables &t, bool fp64, long long pid_begin,
                             long long n, int num_sms, cudaStream_t stream) {
+    launches = 0;
     if (p.ftd > 255 || p.ffd > 255 || p.hd > 32767) return cudaErrorInvalidValue;
     fp64_ = fp64;
     mode_ = instance_mode(p, t);

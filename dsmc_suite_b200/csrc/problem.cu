@@ -99,8 +99,7 @@ struct Uploader {
                                   : cudaMallocAsync(p, bytes, stream);
         if (e == cudaErrorMemoryAllocation && !async && !pr.spare.empty()) {
             cudaGetLastError();   // room taken by blocks that did not fit
-            for (const Problem::Block &q : pr.spare) cudaFree(q.p);
-            pr.spare.clear();
+            pr.release_spare();
             e = cudaMalloc(p, bytes);
         }
         if (e != cudaSuccess)
@@ -144,11 +143,15 @@ void Problem::release() {
         if (async_alloc) cudaFreeAsync(q.p, stream);
         else cudaFree(q.p);
     }
-    for (const Block &q : spare) cudaFree(q.p);
+    release_spare();
     owned.clear();
-    spare.clear();
     bytes = 0;
     t = DevTables{};
+}
+
+void Problem::release_spare() {
+    for (const Block &q : spare) cudaFree(q.p);
+    spare.clear();
 }
 
 void Problem::recycle() {

@@ -33,6 +33,7 @@ struct Problem {
     // and remapped memory.
     void release();
     void recycle();
+    void release_spare();
     static constexpr size_t kSpareBytes = size_t(128) << 20;
 };
 

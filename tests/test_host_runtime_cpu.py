@@ -152,3 +152,38 @@ def test_large_thermal_solves_keep_their_device_block(fake, context, N):
         context.fit_hist(np.ones((50, 8), dtype=np.uint64), 25.0, 3)
         context.thermal(7, 9)
     assert fake.fake_allocs() == before and fake.fake_held() == held
+
+
+@pytest.mark.parametrize("call", ["rows", "solve", "solve64", "setup", "fit"])
+def test_kept_blocks_make_room_when_memory_is_short(fake, N, problem, call):
+    """A context that keeps spare blocks and scratch gives them back before a call of its own fails for
+    want of the memory that they hold."""
+    from dsmc_suite_b200 import Context
+    p, surface = problem
+    wide = p.copy()
+    wide.n_speed_bins = 200   # 83 MB of histograms
+    with Context(0) as ctx:
+        ctx.setup(wide, surface)
+        ctx.setup(p, surface)                                        # the histograms' block is spare
+        ctx.fit_hist(np.ones((400_000, 60), dtype=np.uint64), 25.0, 3)   # 230 MB of scratch
+        do = {
+            "rows": lambda: ctx.enable_particle_outputs(3_000_000),                    # 252 MB
+            "solve": lambda: ctx.run(N.PATH_FAST_FP32, 0, 100),                        # 14 MB
+            "solve64": lambda: ctx.run(N.PATH_FAST_FP64, 0, 100),
+            "setup": lambda: (setattr(wide, "n_speed_bins", 600), ctx.setup(wide, surface)),  # 249 MB
+            "fit": lambda: ctx.fit_hist(np.ones((500_000, 60), dtype=np.uint64), 25.0, 3),    # 294 MB
+        }[call]
+        assert fake.fake_held() > 300_000_000
+        fake.fake_limit(fake.fake_held() + (1 << 20))
+        do()
+
+
+def test_a_solve_too_large_for_the_memory_is_refused_once(fake, context, N, problem):
+    """With nothing left to give back the call reports the lack of memory, and does so without a
+    launch."""
+    context.setup(*problem)
+    fake.fake_limit(fake.fake_held() + (1 << 20))
+    assert N.lib().dsmc_run(context.h, N.PATH_FAST_FP32, 0, 100) == -4
+    assert fake.fake_loops() == 0
+    with pytest.raises(N.DsmcError):
+        context.enable_particle_outputs(1_000_000)
