@@ -130,10 +130,11 @@ int dsmc_run(dsmc_ctx *ctx, int path, int64_t pid_begin, int64_t n);
 int dsmc_sync(dsmc_ctx *ctx);
 
 /* Launch shape of the FAST paths: threads per block, resident blocks per SM (0 = as many as
- * fit), Verlet steps per slot per launch, and launches per captured CUDA graph (served rounds
- * only: a solve's launches carry its parameters and are issued one by one). Results do not depend
- * on the shape: every particle's trajectory is a function of its id and the deposits are integer
- * sums. */
+ * fit), Verlet steps per slot per launch, and launches per round: a served round is one captured
+ * CUDA graph of them; a solve, whose launches carry its parameters, issues them one by one and looks
+ * at its work queue after each round, or after 8192 steps where that comes first. Results do not
+ * depend on the shape: every particle's trajectory is a function of its id and the deposits are
+ * integer sums. */
 int dsmc_set_launch_shape(dsmc_ctx *ctx, int block, int blocks_per_sm, int steps_per_launch,
                           int launches_per_graph);
 /* Kernel launches issued by the last dsmc_run and the resident slot count of the FAST paths. */

@@ -187,3 +187,17 @@ def test_a_solve_too_large_for_the_memory_is_refused_once(fake, context, N, prob
     assert fake.fake_loops() == 0
     with pytest.raises(N.DsmcError):
         context.enable_particle_outputs(1_000_000)
+
+
+@pytest.mark.parametrize("K,G,group", [(64, 16, 16), (1024, 8, 8), (1024, 100, 8), (8192, 8, 1), (100_000, 8, 1), (64, 1, 1)])
+def test_short_launches_are_issued_in_groups(fake, context, N, problem, K, G, group):
+    """A solve looks at its counters once for every launches_per_graph launches, but no later than after
+    the 8192 steps of the default launch; the default shape looks after each launch."""
+    context.set_launch_shape(128, 5, K, G)
+    context.setup(*problem)
+    for n in (100, 1_000_000):   # fewer particles than slots, and more
+        fake.fake_reset()
+        fake.fake_finish_after(6 * group)
+        context.run(N.PATH_FAST_FP32, 0, n)
+        rounds = fake.fake_reads()
+        assert 6 <= rounds <= 7 and fake.fake_loops() == group * rounds == context.launch_info()[0]
