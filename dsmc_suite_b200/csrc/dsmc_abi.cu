@@ -723,7 +723,8 @@ int dsmc_thermal_solve_host(dsmc_ctx *c, int ftd, int ffd, const ThermalParams *
     }
     for (int i = 0; i < h; i++) rcp[i] = 1.0 / piv[i];
     const size_t words = in.size() + 2 * ncol * hh + ncol;
-    if (words > (size_t(1) << 30)) return fail(c, DSMC_ERR_INVALID, "thermal grid too large (%zu doubles)", words);
+    if (words - hh > (size_t(1) << 30))   // the reciprocals aside
+        return fail(c, DSMC_ERR_INVALID, "thermal grid too large (%zu doubles)", words);
     ScratchUse use(c);
     if ((rc = need_scratch(c, words * sizeof(double))) != DSMC_OK) return rc;
     c->scratch_keep = std::max(c->scratch_keep, words * sizeof(double));

@@ -201,3 +201,16 @@ def test_short_launches_are_issued_in_groups(fake, context, N, problem, K, G, gr
         context.run(N.PATH_FAST_FP32, 0, n)
         rounds = fake.fake_reads()
         assert 6 <= rounds <= 7 and fake.fake_loops() == group * rounds == context.launch_info()[0]
+
+
+def test_thermal_grids_up_to_the_limit(fake, context, N):
+    """Inputs, profiles and results of 2^30 doubles are accepted: 3 ncol + 2 h + 2 ncol h, to the depth."""
+    tp = N.ThermalParams.default()
+    tp.n_substep = 1
+    dr = np.sqrt(0.1 * 2.0 * (9.07417 * 3600.0 / 100) * tp.conductivity / tp.density / tp.Cp)
+    most = (2**30 - 3 * 1000) // (2 + 2 * 1000)
+    tp.depth = dr * (most - 0.5)
+    assert context.thermal(10, 100, tp)[1] == most
+    tp.depth = dr * (most + 0.5)
+    with pytest.raises(N.DsmcError, match="too large"):
+        context.thermal(10, 100, tp)
