@@ -135,7 +135,7 @@ struct HotT {
     R run_w;                   // weight-steps deposited in cell ci, not yet flushed
     R W;                       // current weight: exact W0 2^(-c n_day) at cell changes and
                                // events, times 2^(-c) per day-side step in between
-    int hist_key, hist_cnt;
+    int hist_key, hist_cnt;    // speed bin of the histogram's run in cell ci (-1 = none), its steps
     int inst;                  // -1 = empty slot
 };
 using Hot = HotT<float>;
@@ -382,10 +382,13 @@ __device__ __forceinline__ void flush_cell(const FastInst &I, HotT<R> &h) {
     h.run_w = R(0);
 }
 
+// Adds the histogram's run to its bin, before the cell changes: cell x bins alone may take 64 bits
+// (255 x 255 x 34 cells of 1024 bins are 2.26e9 entries).
 template <typename R>
 __device__ __forceinline__ void flush_hist(const FastInst &I, HotT<R> &h) {
     if (h.hist_key >= 0 && h.hist_cnt)
-        atomicAdd(&I.t.speed_hist[h.hist_key], static_cast<unsigned long long>(h.hist_cnt));
+        atomicAdd(&I.t.speed_hist[static_cast<long long>(h.ci) * I.p.n_speed_bins + h.hist_key],
+                  static_cast<unsigned long long>(h.hist_cnt));
     h.hist_key = -1;
     h.hist_cnt = 0;
 }
@@ -429,8 +432,8 @@ __device__ __forceinline__ R c_day_of(const FastInst &I) {
 // one table load. Same cells as track_shell / track_angles. in_r, in_t, in_f are the step's own
 // inside tests per coordinate; only the coordinates that failed are walked (7 % faster on
 // the 1e8-particle Ceres-like workload than walking all three, identical cells). Returns whether
-// the cell changed.
-template <bool kNoBg, class T, typename R>
+// the cell changed. kNoBg: no collision rate to look up. kHist: a speed histogram's run may be open.
+template <bool kNoBg, bool kHist, class T, typename R>
 __device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &b, R x, R y,
                                           R r2, R zz, bool in_r, bool in_t, bool in_f) {
     const FastInst &I = tab.I;
@@ -497,6 +500,7 @@ __device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &
     }
     const int cell = pack_cell(ht, td, fd);
     if (cell == h.cell) return false;
+    if (kHist) flush_hist(I, h);
     // the run of a flying particle has a cell and no negative weight: flushed without the tests
     // of flush_cell (a run of zero adds zero)
     atomicAdd(&I.t.density[h.ci], fixed_of(h.run_w));
@@ -933,6 +937,7 @@ __device__ __forceinline__ int hop_top(const A &a, long long i, const FastInst &
     // kernel launches begin or end (the launch changes neither w0 nor the day count)
     h.W = W;
     const TabOf<A, R> tab{I};
+    if (Mode<kMode>::kAny || Mode<kMode>::kHist) flush_hist(I, h);
     if (first)
         enter_cell(tab, h, b, cell_from_scratch(tab, pos(h, 0), pos(h, 1), pos(h, 2)));
     else
@@ -1372,16 +1377,16 @@ __device__ __forceinline__ void verlet_step(HotT<double> &h, PosT<double> &q, do
 // Event gathering (see fast_kernel): Verlet steps per chunk between the warp's votes.
 constexpr int kChunk = 32;
 
-// Adds the step to the speed histogram's run of (cell, bin).
+// Adds the step to the speed histogram's run of one bin in the current cell.
 template <typename R>
 __device__ __forceinline__ void count_speed(const FastInst &I, const StepConst<R> &k, HotT<R> &h) {
     const R sp = sqrt(fma_r(h.vh[0], h.vh[0], fma_r(h.vh[1], h.vh[1], h.vh[2] * h.vh[2])));
-    const int key = h.ci * k.nbins + min(static_cast<int>(static_cast<float>(sp) * k.inv_bw), k.nbins - 1);
-    if (key == h.hist_key) {
+    const int bin = min(static_cast<int>(static_cast<float>(sp) * k.inv_bw), k.nbins - 1);
+    if (bin == h.hist_key) {
         h.hist_cnt++;
     } else {
         flush_hist(I, h);
-        h.hist_key = key;
+        h.hist_key = bin;
         h.hist_cnt = 1;
     }
 }
@@ -1529,7 +1534,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                if (!move_cell<true, false>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
                     q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
@@ -1561,7 +1566,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<!M::kAny && !M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f) &&
+                if (!move_cell<!M::kAny && !M::kCol, M::kAny || M::kHist>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f) &&
                     kMode == 1 && q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
@@ -1789,8 +1794,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
                 event = kEvLanded;
             } else if (q.r2 >= k.re2) {
                 event = kEvEscaped;
-            } else if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_shell(q, b),
-                                            in_row(q, b), in_column(q, b)) &&
+            } else if (!move_cell<!M::kCol, false>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_shell(q, b),
+                                                   in_row(q, b), in_column(q, b)) &&
                        kMode == 1 && q.r2 != q.r2) {
                 // to the end of its life, or of this launch: there it waits, as a lane that no
                 // longer flies, with its steps settled
