@@ -63,7 +63,7 @@ struct SlotsT {
     int *cell;               // packed (ht << 16) | (td << 8) | fd
     int *run_cell;           // cell of the register deposit run, -1 = none
     R *run_w;                // weight-steps in run_cell not yet flushed (8-byte slot reserved)
-    int *hist_key;           // speed bin of the histogram run in run_cell, -1 = none
+    int *hist_key;           // speed bin of the histogram's run in run_cell, -1 = none
     int *hist_cnt;
     R *pcol, *pthr;          // accumulated collision probability and its threshold
     int *ncol;

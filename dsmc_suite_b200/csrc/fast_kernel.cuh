@@ -135,7 +135,8 @@ struct HotT {
     R run_w;                   // weight-steps deposited in cell ci, not yet flushed
     R W;                       // current weight: exact W0 2^(-c n_day) at cell changes and
                                // events, times 2^(-c) per day-side step in between
-    int hist_key, hist_cnt;    // speed bin of the histogram's run in cell ci (-1 = none), its steps
+    int hist_key, hist_cnt;    // speed bin of the histogram's run (-1 = none), its steps
+    int hist_ci = -1;               // cell of the run in the general loop; in the histogram loop it is ci
     int inst;                  // -1 = empty slot
 };
 using Hot = HotT<float>;
@@ -382,12 +383,12 @@ __device__ __forceinline__ void flush_cell(const FastInst &I, HotT<R> &h) {
     h.run_w = R(0);
 }
 
-// Adds the histogram's run to its bin, before the cell changes: cell x bins alone may take 64 bits
-// (255 x 255 x 34 cells of 1024 bins are 2.26e9 entries).
+// Adds the histogram's run to its bin of cell ci, the run's: cell x bins may take more than 31 bits (255 x
+// 255 x 34 cells of 1024 bins are 2.26e9 entries), so the index is formed here.
 template <typename R>
-__device__ __forceinline__ void flush_hist(const FastInst &I, HotT<R> &h) {
+__device__ __forceinline__ void flush_hist(const FastInst &I, HotT<R> &h, int ci) {
     if (h.hist_key >= 0 && h.hist_cnt)
-        atomicAdd(&I.t.speed_hist[static_cast<long long>(h.ci) * I.p.n_speed_bins + h.hist_key],
+        atomicAdd(&I.t.speed_hist[static_cast<long long>(ci) * I.p.n_speed_bins + h.hist_key],
                   static_cast<unsigned long long>(h.hist_cnt));
     h.hist_key = -1;
     h.hist_cnt = 0;
@@ -432,8 +433,8 @@ __device__ __forceinline__ R c_day_of(const FastInst &I) {
 // one table load. Same cells as track_shell / track_angles. in_r, in_t, in_f are the step's own
 // inside tests per coordinate; only the coordinates that failed are walked (7 % faster on
 // the 1e8-particle Ceres-like workload than walking all three, identical cells). Returns whether
-// the cell changed. kNoBg: no collision rate to look up. kHist: a speed histogram's run may be open.
-template <bool kNoBg, bool kHist, class T, typename R>
+// the cell changed.
+template <bool kNoBg, class T, typename R>
 __device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &b, R x, R y,
                                           R r2, R zz, bool in_r, bool in_t, bool in_f) {
     const FastInst &I = tab.I;
@@ -500,7 +501,6 @@ __device__ __forceinline__ bool move_cell(const T &tab, HotT<R> &h, BoundsT<R> &
     }
     const int cell = pack_cell(ht, td, fd);
     if (cell == h.cell) return false;
-    if (kHist) flush_hist(I, h);
     // the run of a flying particle has a cell and no negative weight: flushed without the tests
     // of flush_cell (a run of zero adds zero)
     atomicAdd(&I.t.density[h.ci], fixed_of(h.run_w));
@@ -937,7 +937,7 @@ __device__ __forceinline__ int hop_top(const A &a, long long i, const FastInst &
     // kernel launches begin or end (the launch changes neither w0 nor the day count)
     h.W = W;
     const TabOf<A, R> tab{I};
-    if (Mode<kMode>::kAny || Mode<kMode>::kHist) flush_hist(I, h);
+    if (Mode<kMode>::kHist) flush_hist(I, h, h.ci);
     if (first)
         enter_cell(tab, h, b, cell_from_scratch(tab, pos(h, 0), pos(h, 1), pos(h, 2)));
     else
@@ -1063,7 +1063,7 @@ __device__ __forceinline__ int land(const A &a, long long i, const FastInst &I, 
 
 // End of a particle's life: per-particle rows (layout of ballistic.c:120,273-276 and
 // advanced.c:262-267,439-444), counters, deposits flushed.
-template <class A, typename R>
+template <int kMode, class A, typename R>
 __device__ __forceinline__ void finish(const A &a, long long i, const FastInst &I, HotT<R> &h,
                        StatAcc &st, int fate) {
     const dsmc_params &p = I.p;
@@ -1094,7 +1094,7 @@ __device__ __forceinline__ void finish(const A &a, long long i, const FastInst &
     st.collisions += ncol;
     if (fate == DSMC_FATE_ESCAPED) st.escaped++;
     flush_cell(I, h);
-    flush_hist(I, h);
+    if (Mode<kMode>::kAny || Mode<kMode>::kHist) flush_hist(I, h, Mode<kMode>::kAny ? h.hist_ci : h.ci);
     h.ci = -1;
     h.inst = -1;
 }
@@ -1276,7 +1276,7 @@ __device__ __forceinline__ bool start_next(const A &a, long long i, HotT<R> &h, 
         const FastInst &I = a.inst(h.inst);
         const int fate = hop_top<kMode>(a, i, I, h, b, st, thi, fi, local_T, true);
         if (fate == 0) return true;
-        finish(a, i, I, h, st, fate);
+        finish<kMode>(a, i, I, h, st, fate);
     }
     return false;
 }
@@ -1377,15 +1377,20 @@ __device__ __forceinline__ void verlet_step(HotT<double> &h, PosT<double> &q, do
 // Event gathering (see fast_kernel): Verlet steps per chunk between the warp's votes.
 constexpr int kChunk = 32;
 
-// Adds the step to the speed histogram's run of one bin in the current cell.
+// Adds the step to the speed histogram's run of one bin in one cell; `from` is the run's cell. The
+// histogram loop (mode 4) counts every step, so the run's cell is the one the step started in; in the
+// general loop a step may count nothing, so the cell is kept beside the run and the run is settled at
+// the end of a launch (the slots have no room for it). 1e6 Ceres-like particles: 41.6 and 62.8 ms, the
+// time of runs under a 32-bit index of cell and bin; with the run settled by the cell walk 42.4 and
+// 63.7 ms, with a 64-bit index 43.3 and 63.3 ms.
 template <typename R>
-__device__ __forceinline__ void count_speed(const FastInst &I, const StepConst<R> &k, HotT<R> &h) {
+__device__ __forceinline__ void count_speed(const FastInst &I, const StepConst<R> &k, HotT<R> &h, int from) {
     const R sp = sqrt(fma_r(h.vh[0], h.vh[0], fma_r(h.vh[1], h.vh[1], h.vh[2] * h.vh[2])));
     const int bin = min(static_cast<int>(static_cast<float>(sp) * k.inv_bw), k.nbins - 1);
-    if (bin == h.hist_key) {
+    if ((bin == h.hist_key) & (from == h.ci)) {
         h.hist_cnt++;
     } else {
-        flush_hist(I, h);
+        flush_hist(I, h, from);
         h.hist_key = bin;
         h.hist_cnt = 1;
     }
@@ -1534,7 +1539,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<true, false>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
+                if (!move_cell<true>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_r, in_t, in_f) &&
                     q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
@@ -1553,6 +1558,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                 h.steps++;
                 h.hop++;
             }
+            const int from = h.ci;
             const R zz = q.z * fabs(q.z);
             const bool in_r = (q.r2 > b.r2lo) & (q.r2 <= b.r2hi);
             const bool in_t = (zz > q.r2 * b.zlo) & (zz <= q.r2 * b.zhi);
@@ -1566,7 +1572,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                     event = 2;
                     break;
                 }
-                if (!move_cell<!M::kAny && !M::kCol, M::kAny || M::kHist>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f) &&
+                if (!move_cell<!M::kAny && !M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, zz, in_r, in_t, in_f) &&
                     kMode == 1 && q.r2 != q.r2) {
                     taken = drift_nowhere(h, taken, n);
                     break;
@@ -1598,7 +1604,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                 if (!collided) {
                     h.run_w += h.W;
                     if (M::kHist || (M::kAny && (k.flags & kFlagHist))) {
-                        count_speed(I, k, h);
+                        count_speed(I, k, h, M::kHist ? from : h.hist_ci);
+                        if (M::kAny) h.hist_ci = h.ci;
                     }
                 }
             }
@@ -1636,11 +1643,12 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                 if (fate == 0) fate = hop_top<kMode>(a, i, I, h, b, st, thi, fi, local_T, false);
             }
             if (fate) {
-                finish(a, i, I, h, st, fate);
+                finish<kMode>(a, i, I, h, st, fate);
                 alive = start_next<kMode>(a, i, h, b, st);
             }
         }
     }
+    if (M::kAny && h.inst >= 0) flush_hist(a.inst(h.inst), h, h.hist_ci);
     if (i >= 0) store_hot(a.s, i, a.nslots, h);
     // statistics of this launch, per instance; the finished count also drives the host loop
     const unsigned fin = st.finished;
@@ -1730,7 +1738,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
                         bool first = false;
                         for (;;) {
                             if (fate) {
-                                if (fate > 0) finish(a, i, I, h, st, fate);
+                                if (fate > 0) finish<kMode>(a, i, I, h, st, fate);
                                 flying = take_next<kMode>(a, i, h, st, thi, fi, local_T);
                                 if (!flying) break;
                                 first = true;
@@ -1794,8 +1802,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) warp_kernel(const __g
                 event = kEvLanded;
             } else if (q.r2 >= k.re2) {
                 event = kEvEscaped;
-            } else if (!move_cell<!M::kCol, false>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_shell(q, b),
-                                                   in_row(q, b), in_column(q, b)) &&
+            } else if (!move_cell<!M::kCol>(Tab{I}, h, b, q.x, q.y, q.r2, q.z * fabs(q.z), in_shell(q, b),
+                                            in_row(q, b), in_column(q, b)) &&
                        kMode == 1 && q.r2 != q.r2) {
                 // to the end of its life, or of this launch: there it waits, as a lane that no
                 // longer flies, with its steps settled
