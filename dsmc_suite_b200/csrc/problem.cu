@@ -79,10 +79,11 @@ struct Uploader {
     int alloc(void **p, size_t bytes) {
         size_t held = bytes;
         if (!async) {
-            // the smallest spare block that fits without wasting more than it holds
+            // the smallest spare block that fits without wasting more than it holds, or 16 MB
+            const size_t most = bytes + std::min(bytes, size_t(16) << 20) + 4096;
             size_t best = pr.spare.size();
             for (size_t k = 0; k < pr.spare.size(); k++)
-                if (pr.spare[k].bytes >= bytes && pr.spare[k].bytes <= 2 * bytes + 4096 &&
+                if (pr.spare[k].bytes >= bytes && pr.spare[k].bytes <= most &&
                     (best == pr.spare.size() || pr.spare[k].bytes < pr.spare[best].bytes))
                     best = k;
             if (best < pr.spare.size()) {

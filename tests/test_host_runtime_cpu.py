@@ -178,6 +178,24 @@ def test_kept_blocks_make_room_when_memory_is_short(fake, N, problem, call):
         do()
 
 
+def test_a_setup_takes_over_blocks_of_about_its_size(fake, context, N, problem):
+    """A block of an earlier problem that is taken over may be larger than asked for, by 16 MB at most."""
+    p, surface = problem
+    wide = p.copy()
+    cells = p.hd * p.ftd * p.ffd
+    for bins in (200, 150, 130, 60, 58):
+        wide.n_speed_bins = bins
+        context.setup(wide, surface)
+        spare = fake.fake_held()
+        context.setup(wide, surface)      # the spare blocks too large for it stay spare, within their bound
+        assert fake.fake_held() == spare
+        fake.fake_limit(fake.fake_held())
+        with pytest.raises(N.DsmcError):  # gives every spare block back, and fails
+            context.enable_particle_outputs(10_000_000)
+        fake.fake_limit(1 << 36)
+        assert fake.fake_held() < cells * (bins + 2) * 8 + (20 << 20)
+
+
 def test_a_solve_too_large_for_the_memory_is_refused_once(fake, context, N, problem):
     """With nothing left to give back the call reports the lack of memory, and does so without a
     launch."""
