@@ -179,6 +179,10 @@ struct ScratchUse {
         c->scratch = nullptr;
         c->scratch_bytes = 0;
     }
+    void clear() {
+        start.clear();
+        total = 0;
+    }
     void part(size_t bytes) {
         start.push_back(total);
         total += (bytes + 255) & ~size_t(255);
@@ -791,17 +795,22 @@ int dsmc_velocity_record(dsmc_ctx *c, int64_t n, int per_bucket, int64_t total_c
     if (rc != DSMC_OK) return rc;
     const int hd = c->params.hd;
     const long long nb = static_cast<long long>(c->params.ftd) * hd;
-    // Chunk of particles whose per-bucket counter rows fit in ~256 MB (a chunk takes as long as its
-    // longest-lived particle, so few large ones).
-    long long chunk = (256ll << 20) / (4 * nb);
-    chunk = chunk < 256 ? 256 : chunk;
-    if (chunk > n) chunk = n > 0 ? n : 1;
+    // Chunk of particles whose per-bucket counter rows fit in 256 MB (a chunk takes as long as its
+    // longest-lived particle, so few large ones), or in 64 MB where memory is short.
     const long long slots = nb * per_bucket;
+    long long chunk = 0;
     ScratchUse use(c);
-    for (size_t bytes : {chunk * nb * sizeof(int), nb * sizeof(int), slots * 3 * sizeof(double), slots * sizeof(int),
-                         slots * sizeof(unsigned long long), chunk * sizeof(int)})
-        use.part(bytes);
-    if ((rc = need_scratch(c, use.total)) != DSMC_OK) return rc;
+    for (const long long room : {256ll << 20, 64ll << 20}) {
+        chunk = std::max(256ll, room / (4 * nb));
+        if (chunk > n) chunk = n > 0 ? n : 1;
+        use.clear();
+        for (size_t bytes : {chunk * nb * sizeof(int), nb * sizeof(int), slots * 3 * sizeof(double), slots * sizeof(int),
+                             slots * sizeof(unsigned long long), chunk * sizeof(int)})
+            use.part(bytes);
+        if ((rc = need_scratch(c, use.total)) != DSMC_ERR_NO_MEMORY) break;
+        cudaGetLastError();
+    }
+    if (rc != DSMC_OK) return rc;
     struct { void *p[6]; } b = {{use.at(0), use.at(1), use.at(2), use.at(3), use.at(4), use.at(5)}};
     DSMC_CUDA_TRY(c, cudaMemsetAsync(b.p[1], 0, nb * sizeof(int), c->stream));
     dsmc::RecordArgs ra{};

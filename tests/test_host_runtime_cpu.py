@@ -154,7 +154,7 @@ def test_large_thermal_solves_keep_their_device_block(fake, context, N):
     assert fake.fake_allocs() == before and fake.fake_held() == held
 
 
-@pytest.mark.parametrize("call", ["rows", "solve", "solve64", "setup", "fit"])
+@pytest.mark.parametrize("call", ["rows", "solve", "solve64", "setup", "fit", "record"])
 def test_kept_blocks_make_room_when_memory_is_short(fake, N, problem, call):
     """A context that keeps spare blocks and scratch gives them back before a call of its own fails for
     want of the memory that they hold."""
@@ -171,10 +171,11 @@ def test_kept_blocks_make_room_when_memory_is_short(fake, N, problem, call):
             "solve": lambda: ctx.run(N.PATH_FAST_FP32, 0, 100),                        # 14 MB
             "solve64": lambda: ctx.run(N.PATH_FAST_FP64, 0, 100),
             "setup": lambda: (setattr(wide, "n_speed_bins", 600), ctx.setup(wide, surface)),  # 249 MB
+            "record": lambda: ctx.velocity_record(200_000, per_bucket=2),   # 256 MB of rows, or 64 MB at a time
             "fit": lambda: ctx.fit_hist(np.ones((500_000, 60), dtype=np.uint64), 25.0, 3),    # 294 MB
         }[call]
         assert fake.fake_held() > 300_000_000
-        fake.fake_limit(fake.fake_held() + (1 << 20))
+        fake.fake_limit(fake.fake_held() + (1 << 20) - (250_000_000 if call == "record" else 0))
         do()
 
 
