@@ -487,16 +487,19 @@ __global__ void __launch_bounds__(128, 4) plain_fp64_kernel(const __grid_constan
 // counts each particle's records below the cap: the replay skips a particle without any and
 // leaves one after its last, so it costs what the first particles of each bucket cost (a chunk of
 // 5000 reference-model particles: 60 ms for the replay of whole lives, as the count pass).
+// A cursor stays at the cap once it is there: the visits of a bucket may be more than an int holds (a
+// chunk is up to 67 million particles, a life 13,000 steps in the mean), and a cursor that wrapped would
+// be below the cap again.
 __global__ void record_scan_kernel(int *rows, int nrows, int nb, int cap, int *todo, int *filled) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
     int run = filled[b];
     for (int q = 0; q < nrows; q++) {
         const long long i = static_cast<long long>(q) * nb + b;
-        const int c = rows[i];
+        const int own = min(rows[i], cap - run);   // its records below the cap
         rows[i] = run;
-        if (c && run < cap) atomicAdd(todo + q, min(c, cap - run));
-        run += c;
+        if (own) atomicAdd(todo + q, own);
+        run += own;
     }
     filled[b] = run;
 }

@@ -54,3 +54,20 @@ def test_velocity_record_with_few_records_per_bucket(ctx, N, O, per_bucket, tota
     keep = keep[:total_cap]
     for a, b in zip(few, full):
         assert np.array_equal(a, b[keep])
+
+
+def test_velocity_record_of_buckets_with_more_than_two_to_the_31_visits(ctx, N):
+    """The first records of a bucket stay its first, however often particles come back to it."""
+    p = N.params_reference(N.RUNNER_BALLISTIC, 6, 12)
+    p.hd, p.unih = 1, p.max_height - p.Radii
+    S = N.SurfaceInputs(T_map=N.latlon_temperature(6, 12, T_ss=235.0, T_floor=150.0))
+    p.n_speed_bins, p.speed_bin_width = 1, 1e6   # one bin: the deposits of each cell
+    n = 2_000_000
+    ctx.solve(N.PATH_PLAIN_FP64, p, S, n)
+    assert ctx.speed_hist().reshape(6, 12).sum(1).max() > 2**31
+    p.n_speed_bins = 0
+    ctx.setup(p, S)
+    few, many = (ctx.velocity_record(m, per_bucket=4) for m in (2000, n))
+    assert len(few[0]) == 6 * 4
+    for a, b in zip(few, many):
+        assert np.array_equal(a, b)
