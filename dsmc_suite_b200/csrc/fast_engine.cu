@@ -515,7 +515,7 @@ cudaError_t FastEngine::run(const dsmc_params &p, const DevTables &t, bool fp64,
     one_ = fp64 || pick_variant(block, blocks_per_sm, mode_) >= 4;
     one_smem_ = one_ ? one_table_bytes(p, fp64) : 0;
     cudaError_t e = ensure_slots(num_sms);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || n <= 0) return e;   // of no particles: nothing issued that a later call would wait for
     e = upload_one(p, t, pid_begin, n, stream);
     if (e != cudaSuccess) return e;
     return drain(n, stream);

@@ -89,6 +89,18 @@ def test_setup_waits_for_its_own_work_alone(fake, context, N, problem):
     assert fake.fake_device_syncs() == 0
 
 
+@pytest.mark.parametrize("path", ["PATH_FAST_FP32", "PATH_FAST_FP64"])
+def test_a_run_of_no_particles_leaves_no_work_behind(fake, context, N, problem, path):
+    """The next set-up, on another stream, takes over the tables that such a run was given."""
+    context.setup(*problem)
+    context.set_stream(fake.fake_stream())
+    context.run(getattr(N, path), 0, 0)
+    assert context.launch_info()[0] == 0
+    context.set_stream(None)
+    context.setup(*problem)
+    assert fake.fake_races() == 0
+
+
 def test_setup_leaves_grids_it_handed_out(fake, context, N, problem):
     """The caller may be reading a grid whose device address it was given, on a stream the context
     does not know: those blocks are freed, which waits for the device, and not written again."""
