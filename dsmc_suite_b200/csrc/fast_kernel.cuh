@@ -136,10 +136,27 @@ struct HotT {
     R W;                       // current weight: exact W0 2^(-c n_day) at cell changes and
                                // events, times 2^(-c) per day-side step in between
     int hist_key, hist_cnt;    // speed bin of the histogram's run (-1 = none), its steps
-    int hist_ci = -1;               // cell of the run in the general loop; in the histogram loop it is ci
     int inst;                  // -1 = empty slot
 };
 using Hot = HotT<float>;
+
+// The general loop's: a step of it may count no speed, so its histogram's run keeps a cell of its own.
+// As a member of HotT it changed ptxas' choices in the lean loops, which have no such run (0 -> 8 B of
+// spill stores at 96 registers): 3e5 Moon-like particles 6.77 -> 6.82 ms, 1e6 Europa-like in FP64 24.9 ->
+// 25.1 ms. So did a finish() that leaves out their empty flush_hist (44 against 24 B in the FP64 loop).
+template <typename R>
+struct GeneralHotT : HotT<R> {
+    int hist_ci = -1;
+};
+template <int kMode, typename R>
+using HotOf = std::conditional_t<Mode<kMode>::kAny, GeneralHotT<R>, HotT<R>>;
+
+// Cell of the histogram's run.
+template <int kMode, typename R>
+__device__ __forceinline__ int &hist_cell(HotT<R> &h) {
+    if constexpr (Mode<kMode>::kAny) return static_cast<GeneralHotT<R> &>(h).hist_ci;
+    else return h.ci;
+}
 
 // Bounds of the current cell: r^2 in (r2lo, r2hi], z|z| in (r^2 zlo, r^2 zhi], longitude between
 // the directions (s0, c0) and (s1, c1).
@@ -1094,7 +1111,7 @@ __device__ __forceinline__ void finish(const A &a, long long i, const FastInst &
     st.collisions += ncol;
     if (fate == DSMC_FATE_ESCAPED) st.escaped++;
     flush_cell(I, h);
-    if (Mode<kMode>::kAny || Mode<kMode>::kHist) flush_hist(I, h, Mode<kMode>::kAny ? h.hist_ci : h.ci);
+    flush_hist(I, h, hist_cell<kMode>(h));
     h.ci = -1;
     h.inst = -1;
 }
@@ -1426,7 +1443,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
     if constexpr (A::kOne) SharedTab<R>::fill(a.one);
     const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long i = a.slot(t);
-    HotT<R> h;
+    HotOf<kMode, R> h;
     if (i >= 0) load_hot(a.s, i, a.nslots, h);
     else h.inst = -1;
     StatAcc st;
@@ -1604,8 +1621,8 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
                 if (!collided) {
                     h.run_w += h.W;
                     if (M::kHist || (M::kAny && (k.flags & kFlagHist))) {
-                        count_speed(I, k, h, M::kHist ? from : h.hist_ci);
-                        if (M::kAny) h.hist_ci = h.ci;
+                        count_speed(I, k, h, M::kHist ? from : hist_cell<kMode>(h));
+                        if (M::kAny) hist_cell<kMode>(h) = h.ci;
                     }
                 }
             }
@@ -1648,7 +1665,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinBlocks) fast_kernel(const __g
             }
         }
     }
-    if (M::kAny && h.inst >= 0) flush_hist(a.inst(h.inst), h, h.hist_ci);
+    if (M::kAny && h.inst >= 0) flush_hist(a.inst(h.inst), h, hist_cell<kMode>(h));
     if (i >= 0) store_hot(a.s, i, a.nslots, h);
     // statistics of this launch, per instance; the finished count also drives the host loop
     const unsigned fin = st.finished;
