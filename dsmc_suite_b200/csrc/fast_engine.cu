@@ -62,10 +62,11 @@ int pick_variant64(int blocks_per_sm, int mode) {
 }
 
 // Variant for a launch shape: blocks_per_sm names the register budget. The default (0) is the
-// fastest measured on B200 for each loop, although ptxas reports spills for all three: the lean
+// fastest measured on B200 for each loop (in the served queue's kernels), spills or not: the lean
 // loop at 96 registers (20 warps per SM) beats 128 registers (16 warps) by 6 % and 80 (24 warps)
 // by 3 %; the collision loop at 96 beats 128 by 1.5 % and 168 (no spills, 12 warps) by 15 %;
-// the general loop at 128 beats 168 by 19 % and 96 by 18 %.
+// the general loop at 128 beats 168 by 19 % and 96 by 18 %. Spill stores by ptxas, served queue and
+// solve of one instance: lean 92 and 0 B, collision 336 and 92 B, general 372 and 40 B.
 int pick_variant(int block, int blocks_per_sm, int mode) {
     if (block > 128) return blocks_per_sm >= 3 ? 1 : 0;
     if (blocks_per_sm == 2) return 3;

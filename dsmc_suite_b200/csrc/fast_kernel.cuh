@@ -72,10 +72,10 @@ __device__ __forceinline__ void accumulate2(float &hx, float &hy, float &lx, flo
 }
 
 // Philox4x32-10 block of the generator's current counter, with the ten rounds kept as a loop: the
-// same words as Philox::next in a fraction of its code. The collision loop takes it in its event
-// paths (launch, start, collision), which run on single lanes: there it cuts ptxas' spill stores
-// from 416 B to 188 B and measured 7 % faster on the 1e7-particle collisional
-// phase 2; the lean and general loops measured
+// same words as Philox::next in a fraction of its code. The config model's collision loop takes it in
+// its event paths (launch, start, collision), which run on single lanes: there it cuts ptxas' spill
+// stores (96 registers: 628 to 336 B in the served queue, 184 to 92 B in a solve of one instance) and
+// measured 7 % faster on the 1e7-particle collisional phase 2; the lean and general loops measured
 // 1-3 % slower with it and keep the unrolled rounds.
 __device__ __forceinline__ void philox_next_rolled(Philox &r) {
     uint32_t c0 = r.pid, c1 = r.event, c2 = r.inst, c3 = 0u, a = r.k0, b = r.k1;
@@ -101,7 +101,9 @@ __device__ __forceinline__ void philox_next(Philox &r) {
     else r.next();
 }
 
-// u in (0, 1): 24 random bits plus half an ulp, so 1 - u and u are never 0.
+// u in (0, 1]: 24 random bits plus half a step, so u is never 0. From 2^23 on the half is rounded away
+// (ties to even), and the top word gives exactly 1: a launch that draws it (1 in 2^24, of either of its
+// two) takes log(1 - u) = -infinity and has an infinite speed; see drift_nowhere.
 __device__ __forceinline__ float unit_open(uint32_t w) {
     return (static_cast<float>(w >> 8) + 0.5f) * (1.0f / 16777216.0f);
 }

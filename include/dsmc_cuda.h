@@ -96,7 +96,11 @@ typedef struct dsmc_ctx dsmc_ctx;
  * at launches and collisions: it follows the same Philox streams as PLAIN_FP64 and differs from
  * it only by rounding, so it serves as the full-size FP64 reference of FAST_FP32. FAST_FP64
  * runs 128-thread blocks, 5 resident per SM in its lean loop (config model, ballistic, no speed
- * histogram), else 4 (3 when asked). */
+ * histogram), else 4 (3 when asked).
+ * Known flaw of FAST_FP32 in the config model: one launch in 8.4 million draws a random number of
+ * exactly 1, whose Maxwellian speed is infinite. Such a particle has no position; it counts as
+ * neither escaped nor bound, deposits its weight into the cell it was launched in until its life
+ * cap, and ends with fate DSMC_FATE_STEP_CAP. */
 enum dsmc_path { DSMC_PATH_PLAIN_FP64 = 0, DSMC_PATH_FAST_FP32 = 1, DSMC_PATH_FAST_FP64 = 2 };
 
 typedef struct dsmc_stats {
@@ -251,7 +255,8 @@ const char *dsmc_noalloc_last_error(void);
 /* Replaces the column loop of thermal_solve (src/thermal/thermal_model.c:105-283): the 1-D heat  */
 /* equation of every surface cell, n_substep implicit steps of one rotation step each, with the  */
 /* surface temperature from the energy balance (solar flux, conduction, thermal emission, H2O    */
-/* sublimation) by bisection and a zero-flux bottom. One GPU thread per (td, fd) column, FP64.   */
+/* sublimation) by bisection and a zero-flux bottom, FP64: eight GPU threads per (td, fd) column */
+/* where all columns fit the SMs' shared memory at once, else one thread per column.             */
 /* flux [ftd][ffd] absorbed flux [W/m^2], or NULL for the reference's analytic flux; writes the  */
 /* surface temperature T_surface [ftd][ffd] and, when h_depth is not NULL, the depth points.     */
 int dsmc_thermal_solve_host(dsmc_ctx *ctx, int ftd, int ffd, const ThermalParams *tp,
