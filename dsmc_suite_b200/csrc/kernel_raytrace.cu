@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -160,9 +161,14 @@ struct Builder {
         nodes[node].first = left;
         nodes[node].count = 0;
         if (depth < 3 && e - b > 2000) {
-            std::thread t([&] { split(left, b, mid, depth + 1); });
+            std::thread t;
+            try {
+                t = std::thread([&] { split(left, b, mid, depth + 1); });
+            } catch (const std::exception &) {   // none to be had: this one builds both
+                split(left, b, mid, depth + 1);
+            }
             split(left + 1, mid, e, depth + 1);
-            t.join();
+            if (t.joinable()) t.join();
         } else {
             split(left, b, mid, depth + 1);
             split(left + 1, mid, e, depth + 1);

@@ -245,3 +245,15 @@ def test_thermal_grids_up_to_the_limit(fake, context, N):
     tp.depth = dr * (most + 0.5)
     with pytest.raises(N.DsmcError, match="too large"):
         context.thermal(10, 100, tp)
+
+
+def test_shadow_flux_without_threads(built, tmp_path):
+    """Subtrees of a mesh are built on threads of their own from 2000 triangles on, where there are any to
+    be had; a process that can make none gets its flux all the same."""
+    from dsmc_suite_b200 import build as B
+    exe = tmp_path / "no_threads"
+    objs = [str(B.OBJ / (s + ".o")) for s in [*B.CUDA_SOURCES, *B.C_SOURCES]]
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I/usr/local/cuda/include", f"-I{ROOT / 'include'}", "-o", str(exe),
+                    str(ROOT / "tests" / "no_threads.cpp"), str(ROOT / "tests" / "fake_cudart.cpp"), *objs, "-lm", "-lpthread"],
+                   check=True, capture_output=True)
+    assert subprocess.run([str(exe)], timeout=60).returncode == 0
